@@ -30,6 +30,12 @@ FO_DEVICE uint32_t cluster_ctarank() {
 FO_DEVICE void cluster_arrive_release() {
   asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
 }
+// Arrive without memory ordering: enough where the barrier only separates phases of execution, or
+// where a narrower fence (mbar_fence_init) has ordered what the others must see.  The release form
+// waits for every global store this thread has in flight.
+FO_DEVICE void cluster_arrive_relaxed() {
+  asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory");
+}
 FO_DEVICE void cluster_wait_acquire() {
   asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
@@ -40,9 +46,11 @@ FO_DEVICE uint32_t mapa_shared(uint32_t smem_addr, uint32_t rank) {
   return r;
 }
 // Arrive on an mbarrier that may live in another CTA of the cluster (address from mapa_shared).
+// Release at CTA scope (the instruction's default): what the barrier hands over is TMEM, ordered by
+// the tcgen05 fence in front of it, and no global data.  At cluster scope the arrive would first
+// wait for every global store this thread has in flight to reach L2 (about 1,500 cycles).
 FO_DEVICE void mbar_arrive_cluster(uint32_t cluster_addr) {
-  asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(cluster_addr)
-               : "memory");
+  asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(cluster_addr) : "memory");
 }
 
 // ------------------------------------------------------------------ mbarrier

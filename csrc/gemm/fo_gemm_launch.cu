@@ -1,5 +1,6 @@
-// Instantiations and host launch code of the tcgen05 GEMM family.
+// Instantiations of the GEMM + collective kernels and the host launch code of the family.
 #include "fo_gemm.h"
+#include "fo_gemm_launch.cuh"
 #include "fo_gemm_sm100.cuh"
 
 #include <mutex>
@@ -30,60 +31,16 @@ EncodeFn get_encode_fn() {
   return fn;
 }
 
-// query != nullptr: do not launch, report the largest co-resident grid instead.
 template <int BN, int STAGES, bool BF16, bool FUSED, bool CTA2, int MT = 1, bool A2A = false, bool NORM = false,
           bool TRACE = false, int EPI = 2>
 cudaError_t launch_one(const GemmTensorMaps* maps, const GemmParams* p, int grid_x, int nvr,
                        bool cooperative, cudaStream_t stream, int* query) {
-  auto kernel = fo_gemm_kernel<BN, STAGES, BF16, FUSED, CTA2, MT, A2A, NORM, TRACE, EPI>;
   constexpr int smem = GemmSmem<BN, STAGES, CTA2, MT, EPI>::kTotalBytes;
   static_assert(smem <= 227 * 1024, "shared memory of this configuration exceeds 227 KB");
   static bool attr_set[16] = {};
-  int dev = 0;
-  cudaGetDevice(&dev);
-  if (dev >= 0 && dev < 16 && !attr_set[dev]) {
-    cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-    if (e != cudaSuccess) return e;
-    attr_set[dev] = true;
-  }
-  cudaLaunchConfig_t cfg = {};
-  cfg.blockDim = dim3(FUSED ? kThreadsFused : kThreadsPlain, 1, 1);
-  cfg.dynamicSmemBytes = smem;
-  cfg.stream = stream;
-  cudaLaunchAttribute attr[2];
-  cfg.attrs = attr;
-  cfg.numAttrs = 0;
-  if (CTA2) {
-    attr[cfg.numAttrs].id = cudaLaunchAttributeClusterDimension;
-    attr[cfg.numAttrs].val.clusterDim.x = 2;
-    attr[cfg.numAttrs].val.clusterDim.y = 1;
-    attr[cfg.numAttrs].val.clusterDim.z = 1;
-    ++cfg.numAttrs;
-  }
-  if (query != nullptr) {
-    cudaDeviceProp prop;
-    cudaError_t e = cudaGetDeviceProperties(&prop, dev);
-    if (e != cudaSuccess) return e;
-    if (!CTA2) {
-      *query = prop.multiProcessorCount;  // shared memory admits exactly one CTA per SM
-      return cudaSuccess;
-    }
-    cfg.gridDim = dim3(prop.multiProcessorCount & ~1, 1, 1);
-    int clusters = 0;
-    e = cudaOccupancyMaxActiveClusters(&clusters, kernel, &cfg);
-    if (e != cudaSuccess) return e;
-    *query = 2 * clusters;
-    return cudaSuccess;
-  }
-  if (CTA2) grid_x &= ~1;
-  if (grid_x < (CTA2 ? 2 : 1)) grid_x = CTA2 ? 2 : 1;
-  cfg.gridDim = dim3(grid_x, nvr, 1);
-  if (cooperative) {
-    attr[cfg.numAttrs].id = cudaLaunchAttributeCooperative;
-    attr[cfg.numAttrs].val.cooperative = 1;
-    ++cfg.numAttrs;
-  }
-  return cudaLaunchKernelEx(&cfg, kernel, *maps, *p);
+  return launch_kernel<CTA2>(fo_gemm_kernel<BN, STAGES, BF16, FUSED, CTA2, MT, A2A, NORM, TRACE, EPI>,
+                             FUSED ? kThreadsFused : kThreadsPlain, smem, attr_set, maps, p, grid_x, nvr, cooperative,
+                             stream, query);
 }
 
 // One case per kernel of gemm/fo_gemm_instances.inc.
@@ -133,12 +90,12 @@ cudaError_t dispatch(int algo, bool bf16, bool fused, const GemmTensorMaps* maps
     if (bf16) return launch_kernel_index<true, true, false, false, true>(kidx, maps, p, grid_x, nvr, coop, s, query);
     return launch_kernel_index<false, true, false, false, true>(kidx, maps, p, grid_x, nvr, coop, s, query);
   }
-  if (bf16) {
-    if (fused) return launch_kernel_index<true, true>(kidx, maps, p, grid_x, nvr, coop, s, query);
-    return launch_kernel_index<true, false>(kidx, maps, p, grid_x, nvr, coop, s, query);
+  if (fused) {
+    if (bf16) return launch_kernel_index<true, true>(kidx, maps, p, grid_x, nvr, coop, s, query);
+    return launch_kernel_index<false, true>(kidx, maps, p, grid_x, nvr, coop, s, query);
   }
-  if (fused) return launch_kernel_index<false, true>(kidx, maps, p, grid_x, nvr, coop, s, query);
-  return launch_kernel_index<false, false>(kidx, maps, p, grid_x, nvr, coop, s, query);
+  if (nvr != 1 || coop) return cudaErrorInvalidConfiguration;
+  return launch_plain_gemm(kidx, bf16, maps, p, grid_x, s, query);
 }
 
 }  // namespace

@@ -36,8 +36,8 @@ struct GemmTensorMaps {
   CUtensorMap b[kMaxVirtualRanks];
   // fused kernels: every rank's staging buffer viewed as [ws * tiles * rows_owned, BN], box
   // (rows_owned x 64): the epilogue's pushes are TMA stores through these.  Pull variant: this
-  // rank's own staging viewed as [tiles * 128, BN], box (128 x 64).  Plain kernels: st[virtual
-  // rank] is the output map of that rank (GemmParams::tma_out), box (128 x 64).
+  // rank's own staging viewed as [tiles * 128, BN], box (128 x 64).  Plain kernels: st[0] is
+  // the output map (GemmParams::tma_out), box (32 x 64).
   CUtensorMap st[kMaxRanks];
 };
 

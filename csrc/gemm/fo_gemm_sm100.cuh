@@ -1,10 +1,6 @@
-// Persistent, warp-specialised tcgen05 GEMM for B200 (sm_100a) with three kinds of epilogue:
+// Persistent, warp-specialised tcgen05 GEMM + collective in one kernel for B200 (sm_100a).  (The
+// GEMM without a collective is in fo_gemm_plain_sm100.cuh.)
 //
-//   * plain      C = A * B^T written row-major, tile-contiguous ("reordered") or row-scattered;
-//   * signalling the same plus a per-wave-group counter bump (and an optional completion-order
-//                monitor) once a tile is globally visible - the producer half of the
-//                counter-gated NCCL path the reference is built around
-//                (reference: src/overlap/gemm_with_signal.h:210-256, :338-361);
 //   * fused      the tile's bf16/fp16 partial sums are pushed, row slice by row slice, straight
 //                into the owning peer GPU's staging buffer over NVLink, the owner's reducer
 //                warps (in the same kernel) sum the `ws` partials in fp32 as soon as every
@@ -21,8 +17,8 @@
 //               (warps 0 and 1 walk their loops with all lanes, waits included, and a lane
 //               chosen by elect.sync issues: warp-uniform control flow lets the compiler keep
 //               counters, addresses and descriptors in uniform registers)
-//   warps 2-5   epilogue: tcgen05.ld -> convert -> swizzled shared-memory transpose ->
-//               128-byte coalesced global (local or peer) stores, then the signal;
+//   warps 2-5   epilogue: tcgen05.ld -> convert -> swizzled shared-memory transpose, then the push
+//               warp's tensor stores or (pull-direct, all-to-all) 128-byte coalesced stores;
 //   warps 6-9   (fused only) reducer for the row slices this rank owns;
 //   warp 10     (fused only) push: one thread turns every finished shared-memory chunk into TMA
 //               stores to the owning ranks' staging memory (or this rank's own, pull protocol)
@@ -47,7 +43,7 @@
 // Worth it when the main loop is long (K per rank in the several thousands).
 //
 // Compile-time variants (template flags; the default builds contain none of their code):
-//   A2A    plain kernel whose epilogue stores each row into the receive buffer of the rank it
+//   A2A    kernel without reducers whose epilogue stores each row into the receive buffer of the rank it
 //          is bound for (fused GEMM + all-to-all), with start- and end-of-call handshakes;
 //   NORM   fused reduce-scatter whose reducers also gather each row's sum of squares and
 //          normalise a 128-row panel when its last tile has been reduced (RMSNorm tail);
@@ -65,8 +61,7 @@
 #include <cuda_runtime.h>
 #include <cstdint>
 
-#include "../common/fo_ptx.cuh"
-#include "fo_gemm_params.h"
+#include "fo_gemm_device.cuh"
 
 namespace fo {
 
@@ -93,87 +88,10 @@ struct GemmSmem {
   static constexpr int kTotalBytes = kMiscOffset + kMiscBytes + 1024;
 };
 
-struct TileCoord {
-  int m, n;
-};
-
-// Position in the launch order -> tile coordinates.  Tiles are swept in column strips
-// `sw` tiles wide, M-major inside a strip; sw == tiles_n gives row-panel-major order.
-__device__ __forceinline__ TileCoord tile_of_position(int pos, int tiles_m, int tiles_n, int sw) {
-  const int per_strip = tiles_m * sw;
-  const int s = pos / per_strip;
-  const int q = pos - s * per_strip;
-  const int w = min(sw, tiles_n - s * sw);
-  TileCoord c;
-  c.m = q / w;
-  c.n = s * sw + (q - c.m * w);
-  return c;
-}
-
-// Wave group of reordered position r: groups are runs of cseg[g] consecutive positions.
-__device__ __forceinline__ void group_of_position(const GemmParams& p, int r, int* g, int* need) {
-  // No grouping, or as many groups as tiles (every group then holds exactly one tile).
-  if (p.num_groups <= 0 || p.cseg == nullptr || p.num_groups == p.num_tiles) {
-    *g = r;
-    *need = 1;
-    return;
-  }
-  int acc = 0, i = 0, n = 1;
-  for (; i < p.num_groups; ++i) {
-    n = p.cseg[i];
-    acc += n;
-    if (r < acc) break;
-  }
-  if (i >= p.num_groups) i = p.num_groups - 1;
-  *g = i;
-  *need = n;
-}
-
-// Reordered position of natural tile t.  A value outside [0, tiles) - a corrupted RA, or one
-// built for another shape - would become an out-of-range address and counter index: it is
-// reported (kStatusBadArgument) and replaced by t, so the kernel stays inside its buffers;
-// the result is then wrong and the status words say why.
-__device__ __forceinline__ int tile_position(const GemmParams& p, int t, int32_t* status) {
-  if (p.RA == nullptr) return t;
-  const int r = p.RA[t];
-  if (static_cast<unsigned>(r) >= static_cast<unsigned>(p.num_tiles)) {
-    ptx::report_status(status, kStatusBadArgument, 1, t, r);
-    return t;
-  }
-  return r;
-}
-
 constexpr int kEpilogueThreads = 128;
 constexpr int kReducerThreads = 128;
 constexpr int kThreadsPlain = 64 + kEpilogueThreads;
 constexpr int kThreadsFused = kThreadsPlain + kReducerThreads + 64;  // + push warp + signal warp
-
-template <bool BF16>
-__device__ __forceinline__ uint32_t pack2(float lo, float hi) {
-  if constexpr (BF16) {
-    __nv_bfloat162 v = __floats2bfloat162_rn(lo, hi);
-    return *reinterpret_cast<uint32_t*>(&v);
-  } else {
-    __half2 v = __floats2half2_rn(lo, hi);
-    return *reinterpret_cast<uint32_t*>(&v);
-  }
-}
-
-template <bool BF16>
-__device__ __forceinline__ void unpack_add(uint32_t w, float& lo, float& hi) {
-  if constexpr (BF16) {
-    __nv_bfloat162 v = *reinterpret_cast<__nv_bfloat162*>(&w);
-    float2 f = __bfloat1622float2(v);
-    lo += f.x;
-    hi += f.y;
-  } else {
-    __half2 v = *reinterpret_cast<__half2*>(&w);
-    float2 f = __half22float2(v);
-    lo += f.x;
-    hi += f.y;
-  }
-}
-
 
 // y = round16(round16(x * scale) * w), the arithmetic of the stand-alone RMSNorm kernels.
 template <bool BF16>
@@ -189,15 +107,6 @@ __device__ __forceinline__ uint32_t norm_scale_mul2(uint32_t x, uint32_t w, floa
     __half2 r = __hmul2(n, *reinterpret_cast<__half2*>(&w));
     return *reinterpret_cast<uint32_t*>(&r);
   }
-}
-
-// round16(a + b) per 16-bit pair, added in fp32: what `a + b` on 16-bit tensors computes.
-template <bool BF16>
-__device__ __forceinline__ uint32_t add2(uint32_t a, uint32_t b) {
-  float lo = 0.f, hi = 0.f;
-  unpack_add<BF16>(a, lo, hi);
-  unpack_add<BF16>(b, lo, hi);
-  return pack2<BF16>(lo, hi);
 }
 
 // Where the reduced vectors of one tile go.  AllReduce: every rank's output (one multimem.st
@@ -446,7 +355,7 @@ __global__ void __launch_bounds__(FUSED ? kThreadsFused : kThreadsPlain, 1)
     }
   };
   static_assert(MT == 1 || (MT == 2 && CTA2 && BN == 256), "two row halves need CTA pairs and BN = 256");
-  static_assert(!(A2A && FUSED), "the all-to-all epilogue is a variant of the plain kernel");
+  static_assert(FUSED != A2A, "either a fused reduction or the all-to-all epilogue");
   static_assert(EPI == 2 || (FUSED && EPI >= 3), "more than two chunk buffers only pay in the fused kernels");
   using L = GemmSmem<BN, STAGES, CTA2, MT, EPI>;
   // Accumulator slots in TMEM: two tiles in flight (MT = 1) or the two halves of one (MT = 2).
@@ -719,11 +628,6 @@ __global__ void __launch_bounds__(FUSED ? kThreadsFused : kThreadsPlain, 1)
     const uint32_t tmem_empty_addr0 =
         CTA2 ? ptx::mapa_shared(ptx::smem_u32(&tmem_empty_bar[0]), 0u) : ptx::smem_u32(&tmem_empty_bar[0]);
 
-    // Plain kernels store finished chunks with TMA (one tensor store per 128 x 64 chunk through
-    // the output map in maps.st[vr]) when the host could describe the output as a 2-D tensor
-    // (row-major and tile-contiguous layouts); the row-scatter and all-to-all modes, whose rows
-    // go to unrelated addresses, keep the per-thread 16-byte stores.
-    const bool use_tma = !FUSED && !A2A && p.tma_out != 0;
     // Fused kernels, pull protocol with direct stores: the partial tile goes to this rank's own
     // staging buffer, so the epilogue threads can store it themselves (as the plain kernels do)
     // instead of handing every chunk to the push warp for a TMA store; the push warp then only
@@ -787,19 +691,8 @@ __global__ void __launch_bounds__(FUSED ? kThreadsFused : kThreadsPlain, 1)
       // 16-byte piece (et & 7) of rows (et >> 3) + 16 * i, i = 0..7.
       uint8_t* row_ptr[8];
       uint32_t row_valid = 0xffu;  // all-to-all: bit i clear = row i has no destination
-      // TMA stores: coordinates of the tile's first chunk in the output's 2-D view
-      int tma_x0 = 0, tma_y0 = 0;
-      if (use_tma) {
-        if (p.out_mode == kOutNatural) {
-          tma_x0 = tc.n * BN;
-          tma_y0 = tc.m * kBM;
-        } else {  // tile-contiguous: [M * N / (rldn * BN)] rows of rldn * BN elements
-          tma_x0 = (r % p.rldn) * BN;
-          tma_y0 = (r / p.rldn) * kBM;
-        }
-      }
 #pragma unroll
-      for (int i = 0; i < 8 && !use_tma; ++i) {
+      for (int i = 0; i < 8; ++i) {
         const int lr = (et >> 3) + 16 * i;
         size_t off = 0;  // element offset of (row lr, tile column 0)
         uint8_t* base = nullptr;
@@ -820,25 +713,6 @@ __global__ void __launch_bounds__(FUSED ? kThreadsFused : kThreadsPlain, 1)
                   static_cast<size_t>(tc.n) * BN;
           } else {
             row_valid &= ~(1u << i);
-          }
-        } else if constexpr (!FUSED) {
-          base = reinterpret_cast<uint8_t*>(p.out[vr]);
-          if (p.out_mode == kOutNatural) {
-            off = (static_cast<size_t>(tc.m) * kBM + lr) * p.N + static_cast<size_t>(tc.n) * BN;
-          } else if (p.out_mode == kOutReorder) {
-            const size_t ld = static_cast<size_t>(p.rldn) * BN;
-            off = static_cast<size_t>(r / p.rldn) * kBM * ld + static_cast<size_t>(r % p.rldn) * BN +
-                  static_cast<size_t>(lr) * ld;
-          } else {  // kOutScatterRows: rows of the [M*N/BN, BN] view are remapped through RE
-            const size_t row_id = static_cast<size_t>(r) * kBM + lr;
-            const int re = p.RE[row_id];
-            if (static_cast<unsigned>(re) >= static_cast<unsigned>(p.M) * static_cast<unsigned>(p.tiles_n)) {
-              // a row index outside the buffer: report it and drop the row
-              ptx::report_status(status, kStatusBadArgument, 2, static_cast<int32_t>(row_id), re);
-              row_valid &= ~(1u << i);
-            } else {
-              off = static_cast<size_t>(re) * BN;
-            }
           }
         }
         row_ptr[i] = base + off * elem + (et & 7) * 16;
@@ -865,13 +739,6 @@ __global__ void __launch_bounds__(FUSED ? kThreadsFused : kThreadsPlain, 1)
           if (!direct && !ptx::mbar_wait_bounded(&chunk_free_bar[chunk_no % EPI], ((chunk_no / EPI) & 1u) ^ 1u,
                                                  s_abort, pipe_timeout)) {
             *s_abort = 1;
-          }
-        }
-        if constexpr (!FUSED && !A2A) {
-          if (use_tma) {
-            // The store issued from this buffer two chunks ago must have read it.
-            if (et == 0) ptx::bulk_wait_group_read<1>();
-            ptx::named_bar_sync(1, kEpilogueThreads);
           }
         }
         const int bsel = (FUSED && !direct) ? static_cast<int>(chunk_no % EPI) : (c & 1);
@@ -915,13 +782,6 @@ __global__ void __launch_bounds__(FUSED ? kThreadsFused : kThreadsPlain, 1)
             ptx::mbar_arrive(&chunk_ready_bar[chunk_no % EPI]);
             ++chunk_no;
           }
-        } else if (use_tma) {
-          ptx::fence_proxy_async_smem();  // generic-proxy writes before the async-proxy read
-          ptx::named_bar_sync(1, kEpilogueThreads);
-          if (et == 0) {
-            ptx::tma_store_2d(&maps.st[vr], epi + (c & 1) * L::kEpiBufBytes, tma_x0 + c * 64, tma_y0);
-            ptx::bulk_commit_group();
-          }
         } else {
           ptx::named_bar_sync(1, kEpilogueThreads);
           const uint8_t* rbuf = epi + (c & 1) * L::kEpiBufBytes;
@@ -950,26 +810,7 @@ __global__ void __launch_bounds__(FUSED ? kThreadsFused : kThreadsPlain, 1)
           ++chunk_no;
         }
       } else {
-        // All of this tile's stores have been issued by every epilogue thread.
-        if (!use_tma) ptx::named_bar_sync(1, kEpilogueThreads);
-        if (et == 0 && p.MM[vr] != nullptr) {
-          int* mm = p.MM[vr];
-          if (use_tma && (p.signal || p.monitor)) {
-            // The tile may be announced only once its tensor stores have been written.
-            ptx::bulk_wait_group<0>();
-            ptx::fence_proxy_async_all();
-          }
-          if (p.signal) {
-            int g, need;
-            group_of_position(p, r, &g, &need);
-            ptx::fence_acq_rel_gpu();
-            ptx::red_release_gpu_add(reinterpret_cast<uint32_t*>(mm + g), 1u);
-          }
-          if (p.monitor) {
-            const int order = atomicAdd(mm + p.mm_stride - 1, 1);
-            mm[p.mm_stride + r] = order;
-          }
-        }
+        ptx::named_bar_sync(1, kEpilogueThreads);  // the chunk buffers are free again
       }
       if (FUSED && et == 0 && p.monitor && p.MM[vr] != nullptr) {
         int* mm = p.MM[vr];
@@ -982,8 +823,6 @@ __global__ void __launch_bounds__(FUSED ? kThreadsFused : kThreadsPlain, 1)
         acc_phase ^= 1u;
       }
     }
-    // No tensor store may still read this CTA's shared memory when the CTA exits.
-    if (use_tma && et == 0) ptx::bulk_wait_group<0>();
     if constexpr (A2A) {
       // End-of-call handshake of the all-to-all: once every CTA of this rank has issued its
       // stores, the last one tells every rank that this rank's rows have been sent and waits

@@ -98,8 +98,8 @@ inline void setup_stage_map(GemmTensorMaps* maps, int rank, void* stage, const G
 }
 
 // Output map of a plain kernel for virtual rank `vr`: the row-major [M, N] output, or the
-// tile-contiguous layout viewed as [M * N / (rldn * BN), rldn * BN], box 128 x 64.  Sets
-// p->tma_out when the layout can be described that way; otherwise the kernel keeps its
+// tile-contiguous layout viewed as [M * N / (rldn * BN), rldn * BN], box 32 x 64 (one epilogue
+// warp's chunk).  Sets p->tma_out when the layout can be described that way; otherwise the kernel keeps its
 // per-thread stores (row-scatter and all-to-all outputs, a tile count that rldn does not divide,
 // an output whose address is not 16-byte aligned).
 inline void setup_out_map(GemmTensorMaps* maps, int vr, void* out, GemmParams* p, int bn) {
@@ -113,7 +113,7 @@ inline void setup_out_map(GemmTensorMaps* maps, int vr, void* out, GemmParams* p
     return;
   }
   const uint64_t rows = static_cast<uint64_t>(p->M) * p->N / cols;
-  const std::string e = encode_tmap_16bit(&maps->st[vr], out, rows, cols, kBM);
+  const std::string e = encode_tmap_16bit(&maps->st[vr], out, rows, cols, 32);
   if (e.empty()) {
     if (vr == 0) p->tma_out = 1;
   } else {

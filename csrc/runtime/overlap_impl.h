@@ -195,7 +195,7 @@ class OverlapImpl : public torch::CustomClassHolder {
 #else
   int64_t opt_validate_ = 0;     // 1: also check the VALUES of RA / RE / cSEG_GPU (a device-to-host copy per call)
 #endif
-  int64_t opt_tma_out_ = -1;     // plain kernels' stores: 1 TMA tensor stores, 0 per-thread stores, -1 by kernel
+  int64_t opt_tma_out_ = -1;     // plain kernels' stores: 0 per-thread stores, else TMA tensor stores where the output allows
   int64_t opt_pull_direct_ = -1;  // pull protocol: epilogue threads store the partials themselves (1), TMA (0), by kernel (-1)
   int64_t opt_wait_sleep_ns_ = 0;   // back-off of the kernel roles that wait with slack (0: poll continuously; measured: no gain)
   int64_t opt_stage_local_ = 0;  // 1: pull protocol (partials staged locally, owners fetch them)
