@@ -28,6 +28,20 @@ cudaError_t launch_gemm(int algo, bool bf16, bool fused, const GemmTensorMaps& m
                         const GemmParams& p, int grid_x, int nvr, bool cooperative,
                         cudaStream_t stream);
 
+// Split over K of a GEMM with few tiles (fo_gemm_splitk_sm100.cuh): `split` CTAs of a cluster per
+// 128 x bn tile; split == 0: none.
+struct SplitChoice {
+  int bn, split;
+};
+constexpr int kMinSplitBlocks = 4;  // k-blocks each CTA of a split must have
+// The split for the problem in `p`, tiled 128 x bn.  Splits are for shapes whose tiles all fit the
+// device several times over; a row-major output may be retiled, a tile-contiguous one keeps `bn`.
+// forced: -1 automatic, 0 never, 2 / 4 / 8 that split wherever it fits the device.
+SplitChoice choose_split(const GemmParams& p, int bn, bool bf16, int forced);
+// `b`: tensor map with boxes of c.bn rows; `p`: tile counts of 128 x c.bn tiles.
+cudaError_t launch_splitk_gemm(SplitChoice c, bool bf16, const CUtensorMap& a, const CUtensorMap& b,
+                               const GemmParams& p, cudaStream_t stream);
+
 // Sets the L2 eviction priorities of the operand loads for the tiling already in `p`: with
 // column strips swept M-major the B strip is re-read by every wave of the strip (keep it: evict
 // last) while A streams through (evict first); with full row panels it is the other way round.

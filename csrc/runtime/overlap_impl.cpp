@@ -116,6 +116,10 @@ void OverlapImpl::SetOption(std::string name, int64_t value) {
   } else if (name == "tma_out") {
     FO_CHECK(value >= -1 && value <= 1, "tma_out must be -1 (automatic), 0 or 1");
     opt_tma_out_ = value;
+  } else if (name == "split_k") {
+    FO_CHECK(value == -1 || value == 0 || value == 2 || value == 4 || value == 8,
+             "split_k must be -1 (automatic), 0 (never), 2, 4 or 8");
+    opt_split_k_ = value;
   } else if (name == "epi_bufs") {
     FO_CHECK(value == 2 || value == 4, "epi_bufs must be 2 or 4");
     opt_epi_bufs_ = value;
@@ -135,6 +139,7 @@ int64_t OverlapImpl::GetOption(std::string name) {
   if (name == "stage_local") return opt_stage_local_;
   if (name == "epi_bufs") return opt_epi_bufs_;
   if (name == "tma_out") return opt_tma_out_;
+  if (name == "split_k") return opt_split_k_;
   if (name == "validate") return opt_validate_;
   if (name == "wait_sleep_ns") return opt_wait_sleep_ns_;
   if (name == "pull_direct") return opt_pull_direct_;
@@ -301,6 +306,16 @@ void OverlapImpl::run_plain(const at::Tensor& A, const at::Tensor& B, void* out,
   p.out[0] = out;
   p.MM[0] = MM;
   p.status[0] = status_.data_ptr<int>();
+  const SplitChoice split = choose_split(p, algo_config(algo).bn, bf16, static_cast<int>(opt_split_k_));
+  if (split.split != 0) {
+    p.tiles_n = p.N / split.bn;
+    p.num_tiles = p.tiles_m * p.tiles_n;
+    if (p.raster_sw > p.tiles_n) p.raster_sw = p.tiles_n;
+    const std::string e = encode_tmap_16bit(&maps.b[0], B.data_ptr(), p.N, p.K, split.bn);
+    FO_CHECK(e.empty(), "B: ", e);
+    cuda_check(launch_splitk_gemm(split, bf16, maps.a[0], maps.b[0], p, stream()), "split-K GEMM launch");
+    return;
+  }
   // TMA tensor stores wherever the output can be described as a 2-D tensor: never slower than the
   // per-thread stores (1024 x 4096 x 1024: 15.3 against 15.6 us for the 256 x 256-per-CTA kernel,
   // 10.0 against 9.9 us for the 128 x 256 one).

@@ -31,6 +31,7 @@ SOURCES = [
     "runtime/loopback.cpp",
     "gemm/fo_gemm_launch.cu",
     "gemm/fo_gemm_plain_launch.cu",
+    "gemm/fo_gemm_splitk_launch.cu",
     "norm/fo_norm.cu",
     "flags/fo_wait.cu",
     "noalloc/fo_noalloc.cu",

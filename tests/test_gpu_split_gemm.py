@@ -1,0 +1,70 @@
+"""The plain GEMM of few output tiles, split over K by the CTAs of a cluster, against fp64."""
+import pytest
+import torch
+
+from flashoverlap_b200 import ops
+from flashoverlap_b200.utils import config, layout
+
+pytestmark = pytest.mark.gpu
+HALF_ULP = {torch.bfloat16: 2.0 ** -9, torch.float16: 2.0 ** -12}
+
+
+@pytest.fixture(scope="module")
+def impl(cuda):
+    i = ops.OverlapImpl()
+    i.nccl_init(0, 1, [0] * 16)
+    i.cutlass_init()
+    return i
+
+
+def _check(c, a, b, dt):
+    """One rounding to the storage type, and fp32 sums of K products: their error is below
+    K * 2^-24 * sum |a b| and, for random signs, far below 2^-18 * sum |a b|."""
+    ref = a.double() @ b.double().t()
+    bound = 2.02 * HALF_ULP[dt] * ref.abs() + 2.0 ** -18 * (a.double().abs() @ b.double().abs().t()) + 2.0 ** -24
+    assert ((c.double() - ref).abs() <= bound).all()
+
+
+# smallest K, a K that no split divides, K with a partial k-block, one tile, the largest tile counts of
+# each split, N that only 128-wide tiles divide
+@pytest.mark.parametrize("dt", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("M,N,K,algo", [(128, 256, 256, 0), (128, 1024, 1000, 1), (128, 8192, 3584, 0), (256, 4096, 1096, 1),
+                                        (128, 1152, 4096, 2), (384, 1280, 72 * 64 + 8, 24), (512, 512, 2048, 3),
+                                        (2176, 1024, 520, 0)])
+def test_split_gemm_natural(cuda, impl, dt, M, N, K, algo):
+    algo = config.default_solution(M, N, algo)["Algo"]
+    a = (torch.randn(M, K, device=cuda) * 0.5).to(dt)
+    b = (torch.randn(N, K, device=cuda) * 0.5).to(dt)
+    try:
+        for split in (-1, 0, 2, 4, 8):
+            impl.set_option("split_k", split)
+            c = torch.full((M, N), float("nan"), device=cuda, dtype=dt)
+            impl.cutlass_gemm(a, b, c, algo)
+            _check(c, a, b, dt)
+            again = torch.empty_like(c)
+            impl.cutlass_gemm(a, b, again, algo)
+            assert torch.equal(c, again)             # the partial sums are added in a fixed order
+    finally:
+        impl.set_option("split_k", -1)
+    impl.check_status()
+
+
+@pytest.mark.parametrize("M,N,K,algo,rldn", [(128, 2048, 1024, 0, 1), (256, 1024, 520, 2, 2), (256, 512, 4096, 1, 1)])
+def test_split_gemm_reordered(cuda, impl, M, N, K, algo, rldn):
+    p = config.algo_params(algo)
+    tm, tn = M // p["BM"], N // p["BN"]
+    dt = torch.bfloat16
+    a = (torch.randn(M, K, device=cuda) * 0.5).to(dt)
+    b = (torch.randn(N, K, device=cuda) * 0.5).to(dt)
+    RA = torch.randperm(tm * tn, device=cuda, dtype=torch.int32)
+    e = torch.empty(0, dtype=torch.int32)
+    mm = torch.zeros(tm + 1, tn, device=cuda, dtype=torch.int32)
+    try:
+        for split in (-1, 2, 4, 8):
+            impl.set_option("split_k", split)
+            c = torch.full((M, N), float("nan"), device=cuda, dtype=dt)
+            impl.gemm_allreduce_overlap(a, b, c, mm, RA, rldn, e, e.to(cuda), algo, False)
+            _check(layout.from_reordered(c.cpu(), M, N, p["BM"], p["BN"], RA.cpu(), rldn).to(cuda), a, b, dt)
+    finally:
+        impl.set_option("split_k", -1)
+    impl.check_status()
