@@ -16,9 +16,9 @@ void cuda_check(cudaError_t e, const char* what) {
 }
 }  // namespace
 
-SymmetricHeap::SymmetricHeap(int rank, int world, ncclComm_t comm, bool loopback)
-    : rank_(rank), world_(world), comm_(comm), loopback_(loopback) {
-  if (world_ > 1 && !loopback_ && comm_ == nullptr) {
+SymmetricHeap::SymmetricHeap(int rank, int world, ncclComm_t comm)
+    : rank_(rank), world_(world), comm_(comm) {
+  if (world_ > 1 && comm_ == nullptr) {
     throw std::runtime_error("SymmetricHeap needs an NCCL communicator to exchange IPC handles");
   }
 }
@@ -28,7 +28,7 @@ SymmetricHeap::~SymmetricHeap() {
     if (!r->owned) continue;
     for (int i = 0; i < static_cast<int>(r->ptr.size()); ++i) {
       if (r->ptr[i] == nullptr) continue;
-      if (r->loopback || i == r->rank) {
+      if (i == r->rank) {
         cudaFree(r->ptr[i]);
       } else {
         cudaIpcCloseMemHandle(r->ptr[i]);
@@ -41,14 +41,11 @@ SymmetricRegion* SymmetricHeap::allocate(size_t bytes, cudaStream_t stream) {
   auto region = std::make_unique<SymmetricRegion>();
   region->bytes = bytes;
   region->rank = rank_;
-  region->loopback = loopback_;
   region->ptr.assign(world_, nullptr);
 
-  if (loopback_ || world_ == 1) {
-    for (int r = 0; r < world_; ++r) {
-      cuda_check(cudaMalloc(&region->ptr[r], bytes), "cudaMalloc(symmetric loopback)");
-      cuda_check(cudaMemsetAsync(region->ptr[r], 0, bytes, stream), "cudaMemsetAsync");
-    }
+  if (world_ == 1) {
+    cuda_check(cudaMalloc(&region->ptr[0], bytes), "cudaMalloc(symmetric)");
+    cuda_check(cudaMemsetAsync(region->ptr[0], 0, bytes, stream), "cudaMemsetAsync");
     cuda_check(cudaStreamSynchronize(stream), "cudaStreamSynchronize");
     regions_.push_back(std::move(region));
     return regions_.back().get();
@@ -95,10 +92,8 @@ void SymmetricHeap::release(SymmetricRegion* region, cudaStream_t stream) {
   }
   if (idx == regions_.size()) return;  // not ours
   if (region->owned) {
-    if (region->loopback || world_ == 1) {
-      for (void* p : region->ptr) {
-        if (p != nullptr) cudaFree(p);
-      }
+    if (world_ == 1) {
+      cudaFree(region->ptr[0]);
     } else {
       for (int r = 0; r < world_; ++r) {
         if (r != rank_ && region->ptr[r] != nullptr) cudaIpcCloseMemHandle(region->ptr[r]);

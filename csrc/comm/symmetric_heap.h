@@ -7,9 +7,6 @@
 // the NCCL communicator the runtime already owns (an all-gather of the 64-byte handles) and
 // opened by the peers with cudaIpcOpenMemHandle.  Allocation is therefore a collective:
 // every rank must allocate the same sizes in the same order.
-//
-// "Loopback" heaps back the single-GPU emulation used by tests: all `world` copies live on
-// the current device and no inter-process exchange happens.
 #pragma once
 #include <cuda_runtime.h>
 #include <nccl.h>
@@ -24,7 +21,6 @@ struct SymmetricRegion {
   size_t bytes = 0;
   int rank = 0;
   std::vector<void*> ptr;  // ptr[r]: rank r's copy as addressable from this process; ptr[rank] is local
-  bool loopback = false;
   bool owned = true;           // false: registered by the caller, never freed here
   void* multicast = nullptr;   // NVSwitch multicast mapping of the buffer, if any
   void* local() const { return ptr[rank]; }
@@ -37,8 +33,8 @@ struct SymmetricRegion {
 
 class SymmetricHeap {
  public:
-  // comm may be null only when world == 1 or loopback is true.
-  SymmetricHeap(int rank, int world, ncclComm_t comm, bool loopback);
+  // comm may be null only when world == 1.
+  SymmetricHeap(int rank, int world, ncclComm_t comm);
   ~SymmetricHeap();
   SymmetricHeap(const SymmetricHeap&) = delete;
   SymmetricHeap& operator=(const SymmetricHeap&) = delete;
@@ -61,12 +57,10 @@ class SymmetricHeap {
   void detach_comm() { comm_ = nullptr; }
   int rank() const { return rank_; }
   int world() const { return world_; }
-  bool loopback() const { return loopback_; }
 
  private:
   int rank_, world_;
   ncclComm_t comm_;
-  bool loopback_;
   std::vector<std::unique_ptr<SymmetricRegion>> regions_;
 };
 

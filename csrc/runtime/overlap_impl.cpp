@@ -58,7 +58,7 @@ void OverlapImpl::NcclInit(int64_t rank, int64_t world, std::vector<int64_t> id)
     ncclUniqueId uid = unpack_nccl_id(id);
     FO_NCCL_CHECK(ncclCommInitRank(&comm_, world_, uid, rank_));
   }
-  heap_ = std::make_shared<SymmetricHeap>(rank_, world_, comm_, false);
+  heap_ = std::make_shared<SymmetricHeap>(rank_, world_, comm_);
   status_ = at::zeros({kStatusWords}, at::TensorOptions().dtype(at::kInt).device(at::kCUDA, device_));
 }
 
