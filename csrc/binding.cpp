@@ -9,6 +9,7 @@
 
 #include "common/fo_check.h"
 #include "comm/nccl_utils.h"
+#include "elementwise/fo_elementwise.h"
 #include "flags/fo_wait.h"
 #include "norm/fo_norm.h"
 #include "runtime/baseline_impl.h"
@@ -76,6 +77,62 @@ void rmsnorm(at::Tensor X, at::Tensor RX, at::Tensor RW, double eps) {
                                     static_cast<float>(eps), bf, sm_count_of_current_device(),
                                     c10::cuda::getCurrentCUDAStream().stream()),
                  "rmsnorm");
+}
+
+bool aligned16(const at::Tensor& t) { return reinterpret_cast<uintptr_t>(t.data_ptr()) % 16 == 0; }
+
+// H = X + T, RX = rmsnorm(H) * RW; H may be X.
+void add_rmsnorm(at::Tensor X, at::Tensor T, at::Tensor H, at::Tensor RX, at::Tensor RW, double eps) {
+  const bool bf = is_bf16(X, "X");
+  is_bf16(T, "T");
+  is_bf16(H, "H");
+  is_bf16(RX, "RX");
+  is_bf16(RW, "RW");
+  FO_CHECK(T.scalar_type() == X.scalar_type() && H.scalar_type() == X.scalar_type() &&
+               RX.scalar_type() == X.scalar_type() && RW.scalar_type() == X.scalar_type(),
+           "X, T, H, RX and RW must share a dtype");
+  FO_CHECK(X.dim() == 2 && T.sizes() == X.sizes() && H.sizes() == X.sizes() && RX.sizes() == X.sizes(),
+           "X, T, H and RX must be [rows, dim]");
+  FO_CHECK(RW.numel() == X.size(1), "RW must have dim elements");
+  FO_CHECK(H.data_ptr() != RX.data_ptr() || X.numel() == 0, "H and RX must not alias");
+  FO_CHECK(aligned16(X) && aligned16(T) && aligned16(H) && aligned16(RX) && aligned16(RW),
+           "all tensors must be 16-byte aligned");
+  c10::cuda::CUDAGuard guard(X.device());
+  fo::cuda_check(fo::add_rmsnorm_launch(X.data_ptr(), T.data_ptr(), H.data_ptr(), RX.data_ptr(), RW.data_ptr(),
+                                        static_cast<int>(X.size(0)), static_cast<int>(X.size(1)),
+                                        static_cast<float>(eps), bf, sm_count_of_current_device(),
+                                        c10::cuda::getCurrentCUDAStream().stream()),
+                 "add_rmsnorm");
+}
+
+// Rotary embedding, in place, of the first `heads` heads of every row of QKV [tokens, row_elems].
+void rope_(at::Tensor QKV, int64_t seq, int64_t heads, int64_t head_dim, double theta) {
+  const bool bf = is_bf16(QKV, "QKV");
+  FO_CHECK(QKV.dim() == 2 && heads >= 0 && head_dim > 0 && heads * head_dim <= QKV.size(1),
+           "QKV must be [tokens, at least heads * head_dim]");
+  FO_CHECK(seq > 0 && head_dim % 8 == 0 && QKV.size(1) % 8 == 0, "head_dim and the row length must be multiples of 8");
+  FO_CHECK(aligned16(QKV), "QKV must be 16-byte aligned");
+  c10::cuda::CUDAGuard guard(QKV.device());
+  fo::cuda_check(fo::rope_launch(QKV.data_ptr(), static_cast<int>(QKV.size(0)), static_cast<int>(seq),
+                                 static_cast<int>(heads), static_cast<int>(head_dim), static_cast<int>(QKV.size(1)),
+                                 static_cast<float>(theta), bf, c10::cuda::getCurrentCUDAStream().stream()),
+                 "rope");
+}
+
+// Y [rows, f] = silu(GU[:, :f]) * GU[:, f:].
+void swiglu(at::Tensor GU, at::Tensor Y) {
+  const bool bf = is_bf16(GU, "GU");
+  is_bf16(Y, "Y");
+  FO_CHECK(Y.scalar_type() == GU.scalar_type(), "GU and Y must share a dtype");
+  FO_CHECK(GU.dim() == 2 && Y.dim() == 2 && Y.size(0) == GU.size(0) && GU.size(1) == 2 * Y.size(1),
+           "GU must be [rows, 2 f] and Y [rows, f]");
+  FO_CHECK(Y.size(1) % 8 == 0, "f must be a multiple of 8");
+  FO_CHECK(aligned16(GU) && aligned16(Y), "GU and Y must be 16-byte aligned");
+  c10::cuda::CUDAGuard guard(GU.device());
+  fo::cuda_check(fo::swiglu_launch(GU.data_ptr(), Y.data_ptr(), static_cast<int>(GU.size(0)),
+                                   static_cast<int>(Y.size(1)), bf, sm_count_of_current_device(),
+                                   c10::cuda::getCurrentCUDAStream().stream()),
+                 "swiglu");
 }
 
 void reorder_impl(at::Tensor X, at::Tensor Y, int64_t rows, int64_t dim, int64_t BM, int64_t BN,
@@ -215,6 +272,9 @@ TORCH_LIBRARY(flashoverlap_op, m) {
   // additions
   m.def("reorder_rmsnorm_eps", &reorder_rmsnorm_eps);
   m.def("rmsnorm", &rmsnorm);
+  m.def("add_rmsnorm", &add_rmsnorm);
+  m.def("rope_", &rope_);
+  m.def("swiglu", &swiglu);
   m.def("reorder", &reorder);
   m.def("unreorder", &unreorder);
   m.def("wait_flag", &wait_flag);

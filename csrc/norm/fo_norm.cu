@@ -1,4 +1,4 @@
-// Memory-bound row kernels: RMSNorm, fused tile-un-reorder + RMSNorm, and the standalone
+// Memory-bound row kernels: RMSNorm, residual add + RMSNorm, fused tile-un-reorder + RMSNorm, and the standalone
 // row-major <-> tile-contiguous reorder.  Counterparts of the reference's
 // reorder_rmsnorm_kernel / rmsnorm_kernel (src/rmsnorm/rmsnorm.cuh:14-117); the standalone
 // reorder has no counterpart there (its layout change only ever happens inside the GEMM
@@ -42,6 +42,19 @@ __device__ __forceinline__ uint32_t scale_mul2(uint32_t x, uint32_t w, float sca
   } else {
     __half2 n = __floats2half2_rn(xf.x * scale, xf.y * scale);
     __half2 r = __hmul2(n, *reinterpret_cast<__half2*>(&w));
+    return *reinterpret_cast<uint32_t*>(&r);
+  }
+}
+
+// round16(a + b) per 16-bit pair, added in fp32: what `a + b` on 16-bit tensors computes.
+template <bool BF16>
+__device__ __forceinline__ uint32_t add2_16(uint32_t a, uint32_t b) {
+  const float2 x = unpack2<BF16>(a), y = unpack2<BF16>(b);
+  if constexpr (BF16) {
+    __nv_bfloat162 r = __floats2bfloat162_rn(x.x + y.x, x.y + y.y);
+    return *reinterpret_cast<uint32_t*>(&r);
+  } else {
+    __half2 r = __floats2half2_rn(x.x + y.x, x.y + y.y);
     return *reinterpret_cast<uint32_t*>(&r);
   }
 }
@@ -163,6 +176,73 @@ __global__ void __launch_bounds__(kNormThreads, (VPT <= 2 ? 6 : (VPT <= 4 ? 4 : 
   }
 }
 
+// H = round16(X + T), Y = rmsnorm(H) * W: the residual add in front of a norm, in the norm's pass over
+// the rows (an add of its own reads two matrices and writes one, and the norm reads that again:
+// 55 us for the two at 4096 x 8192, 46 us here for 268 MB, 5.8 TB/s).
+// H may be X (the residual stream is updated in place) and Y may be X or H, so no pointer is
+// restrict-qualified: a row is read into registers, a whole row ahead, before it is stored, and a
+// thread stores H before Y.  Threads, rows per CTA and prefetch as in rmsnorm_kernel; the weights
+// are re-read from L1 per row, their registers hold the second operand.
+template <bool BF16, int VPT>
+__global__ void __launch_bounds__(kNormThreads, (VPT <= 2 ? 4 : 2))
+    add_rmsnorm_kernel(const uint16_t* X, const uint16_t* T, uint16_t* H, uint16_t* Y, const uint16_t* W, int rows,
+                       int dim, float eps) {
+  __shared__ float red[kNormThreads / 32];
+  const int nvec = dim / 8;
+  const int per_cta = (rows + gridDim.x - 1) / gridDim.x;
+  const int row_begin = blockIdx.x * per_cta;
+  const int row_end = min(rows, row_begin + per_cta);
+  if (row_begin >= row_end) return;
+  auto load_row = [&](int b, uint4 (&x)[VPT], uint4 (&t)[VPT]) {
+    const size_t base = static_cast<size_t>(b) * dim;
+#pragma unroll
+    for (int i = 0; i < VPT; ++i) {
+      const int j = threadIdx.x + i * kNormThreads;
+      if (j < nvec) {
+        x[i] = __ldcs(reinterpret_cast<const uint4*>(X + base + static_cast<size_t>(j) * 8));
+        t[i] = __ldcs(reinterpret_cast<const uint4*>(T + base + static_cast<size_t>(j) * 8));
+      }
+    }
+  };
+  uint4 x[VPT], t[VPT], h[VPT];
+  load_row(row_begin, x, t);
+  for (int b = row_begin; b < row_end; ++b) {
+    const size_t base = static_cast<size_t>(b) * dim;
+    float ss = 0.f;
+#pragma unroll
+    for (int i = 0; i < VPT; ++i) {
+      const int j = threadIdx.x + i * kNormThreads;
+      if (j < nvec) {
+        h[i] = make_uint4(add2_16<BF16>(x[i].x, t[i].x), add2_16<BF16>(x[i].y, t[i].y),
+                          add2_16<BF16>(x[i].z, t[i].z), add2_16<BF16>(x[i].w, t[i].w));
+        const uint32_t* u = reinterpret_cast<const uint32_t*>(&h[i]);
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+          const float2 f = unpack2<BF16>(u[k]);
+          ss += f.x * f.x + f.y * f.y;
+        }
+      }
+    }
+    if (b + 1 < row_end) load_row(b + 1, x, t);
+    ss = block_sum(ss, red);
+    const float scale = rsqrtf(ss / static_cast<float>(dim) + eps);
+#pragma unroll
+    for (int i = 0; i < VPT; ++i) {
+      const int j = threadIdx.x + i * kNormThreads;
+      if (j < nvec) {
+        const uint4 w = __ldg(reinterpret_cast<const uint4*>(W + static_cast<size_t>(j) * 8));
+        uint4 y;
+        y.x = scale_mul2<BF16>(h[i].x, w.x, scale);
+        y.y = scale_mul2<BF16>(h[i].y, w.y, scale);
+        y.z = scale_mul2<BF16>(h[i].z, w.z, scale);
+        y.w = scale_mul2<BF16>(h[i].w, w.w, scale);
+        __stcs(reinterpret_cast<uint4*>(H + base + static_cast<size_t>(j) * 8), h[i]);
+        __stcs(reinterpret_cast<uint4*>(Y + base + static_cast<size_t>(j) * 8), y);
+      }
+    }
+  }
+}
+
 // TO_REORDERED: Y[reordered] = X[natural]; otherwise Y[natural] = X[reordered].
 // Same shape as the norm kernel: each CTA takes a contiguous block of rows, each thread owns VPT
 // 16-byte vectors of a row, the tile look-up through RA is done only when the block of rows
@@ -226,16 +306,44 @@ __global__ void __launch_bounds__(kNormThreads, (VPT <= 2 ? 6 : (VPT <= 4 ? 4 : 
   }
 }
 
+// Contiguous row blocks: enough CTAs to fill the machine several times over, yet a few rows per CTA
+// so that the prefetch and the cached tile look-ups pay off.
+int row_grid(int rows, int sm_count) {
+  int grid = rows < sm_count * 8 ? rows : sm_count * 8;
+  if (rows >= sm_count * 32) grid = (rows + 3) / 4 < sm_count * 16 ? (rows + 3) / 4 : sm_count * 16;
+  return grid < 1 ? 1 : grid;
+}
+
+template <bool BF16>
+cudaError_t launch_add_norm(const void* X, const void* T, void* H, void* Y, const void* W, int rows, int dim,
+                            float eps, int sm_count, cudaStream_t stream) {
+  const int vpt = (dim / 8 + kNormThreads - 1) / kNormThreads;
+  const int grid = row_grid(rows, sm_count);
+  const uint16_t* x = static_cast<const uint16_t*>(X);
+  const uint16_t* t = static_cast<const uint16_t*>(T);
+  uint16_t* h = static_cast<uint16_t*>(H);
+  uint16_t* y = static_cast<uint16_t*>(Y);
+  const uint16_t* w = static_cast<const uint16_t*>(W);
+  if (vpt <= 1) {
+    add_rmsnorm_kernel<BF16, 1><<<grid, kNormThreads, 0, stream>>>(x, t, h, y, w, rows, dim, eps);
+  } else if (vpt <= 2) {
+    add_rmsnorm_kernel<BF16, 2><<<grid, kNormThreads, 0, stream>>>(x, t, h, y, w, rows, dim, eps);
+  } else if (vpt <= 4) {
+    add_rmsnorm_kernel<BF16, 4><<<grid, kNormThreads, 0, stream>>>(x, t, h, y, w, rows, dim, eps);
+  } else if (vpt <= 8) {
+    add_rmsnorm_kernel<BF16, 8><<<grid, kNormThreads, 0, stream>>>(x, t, h, y, w, rows, dim, eps);
+  } else {
+    return cudaErrorInvalidValue;  // dim > 16384
+  }
+  return cudaGetLastError();
+}
+
 template <bool BF16, bool REORDER>
 cudaError_t launch_norm(const void* X, void* Y, const void* W, int rows, int dim, int BM, int BN,
                         int rldn, const int* RA, float eps, int sm_count, cudaStream_t stream) {
   const int nvec = dim / 8;
   const int vpt = (nvec + kNormThreads - 1) / kNormThreads;
-  // contiguous row blocks: enough CTAs to fill the machine several times over, yet a few
-  // rows per CTA so that the prefetch and the cached tile look-ups pay off
-  int grid = rows < sm_count * 8 ? rows : sm_count * 8;
-  if (rows >= sm_count * 32) grid = (rows + 3) / 4 < sm_count * 16 ? (rows + 3) / 4 : sm_count * 16;
-  if (grid < 1) grid = 1;
+  const int grid = row_grid(rows, sm_count);
   const uint16_t* x = static_cast<const uint16_t*>(X);
   uint16_t* y = static_cast<uint16_t*>(Y);
   const uint16_t* w = static_cast<const uint16_t*>(W);
@@ -267,6 +375,14 @@ cudaError_t rmsnorm_launch(const void* X, void* Y, const void* W, int rows, int 
               : launch_norm<false, false>(X, Y, W, rows, dim, 1, 1, 1, nullptr, eps, sm_count, stream);
 }
 
+cudaError_t add_rmsnorm_launch(const void* X, const void* T, void* H, void* Y, const void* W, int rows, int dim,
+                               float eps, bool bf16, int sm_count, cudaStream_t stream) {
+  if (dim % 8 != 0) return cudaErrorInvalidValue;
+  if (rows == 0) return cudaSuccess;
+  return bf16 ? launch_add_norm<true>(X, T, H, Y, W, rows, dim, eps, sm_count, stream)
+              : launch_add_norm<false>(X, T, H, Y, W, rows, dim, eps, sm_count, stream);
+}
+
 cudaError_t reorder_rmsnorm_launch(const void* X, void* Y, const void* W, int rows, int dim, int BM,
                                    int BN, int rldn, const int* RA, float eps, bool bf16,
                                    int sm_count, cudaStream_t stream) {
@@ -284,11 +400,7 @@ cudaError_t reorder_launch(const void* X, void* Y, int rows, int dim, int BM, in
   if (rows == 0) return cudaSuccess;
   const int nvec = dim / 8;
   const int vpt = (nvec + kNormThreads - 1) / kNormThreads;
-  // contiguous row blocks, as for the norm kernels: a few rows per CTA so that the cached tile
-  // look-ups pay off, enough CTAs to fill the machine several times over
-  int grid = rows < sm_count * 8 ? rows : sm_count * 8;
-  if (rows >= sm_count * 32) grid = (rows + 3) / 4 < sm_count * 16 ? (rows + 3) / 4 : sm_count * 16;
-  if (grid < 1) grid = 1;
+  const int grid = row_grid(rows, sm_count);
   const uint16_t* x = static_cast<const uint16_t*>(X);
   uint16_t* y = static_cast<uint16_t*>(Y);
 #define FO_LAUNCH_REORDER(V)                                                                              \

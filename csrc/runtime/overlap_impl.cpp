@@ -625,7 +625,7 @@ void OverlapImpl::GemmReduceScatterAddRmsNormFused(at::Tensor A, at::Tensor B, a
   NvtxRange nvtx_range("flashoverlap::gemm_reducescatter_add_rmsnorm_fused");
   FO_CHECK(heap_ != nullptr, "call nccl_init first");
   if (world_ == 1) {
-    // One rank: nothing to reduce; GEMM, residual add, then the stand-alone RMSNorm.
+    // One rank: nothing to reduce; GEMM, then residual add and RMSNorm in one pass over the rows.
     const GemmShape s = check_operands(A, B);
     FO_CHECK(W.is_cuda() && W.is_contiguous() && W.scalar_type() == A.scalar_type() && W.numel() == s.N,
              "W must be a contiguous CUDA tensor of N elements in the operands' dtype");
@@ -634,10 +634,9 @@ void OverlapImpl::GemmReduceScatterAddRmsNormFused(at::Tensor A, at::Tensor B, a
     at::Tensor tmp = at::empty({s.M, s.N}, A.options());
     Gemm(A, B, tmp, Algo);
     at::Tensor r2 = R.view({s.M, s.N});
-    r2.add_(tmp);
-    cuda_check(rmsnorm_launch(r2.data_ptr(), Y.data_ptr(), W.data_ptr(), s.M, s.N, static_cast<float>(eps), s.bf16,
-                              sm_count_, stream()),
-               "rmsnorm");
+    cuda_check(add_rmsnorm_launch(r2.data_ptr(), tmp.data_ptr(), r2.data_ptr(), Y.data_ptr(), W.data_ptr(), s.M, s.N,
+                                  static_cast<float>(eps), s.bf16, sm_count_, stream()),
+               "add_rmsnorm");
     return;
   }
   run_fused(kCommFusedRS, A, B, R, kOutNatural, nullptr, 1, nullptr, 0, false, nullptr, 0,

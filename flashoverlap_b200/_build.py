@@ -33,6 +33,7 @@ SOURCES = [
     "gemm/fo_gemm_plain_launch.cu",
     "gemm/fo_gemm_splitk_launch.cu",
     "norm/fo_norm.cu",
+    "elementwise/fo_elementwise.cu",
     "flags/fo_wait.cu",
     "noalloc/fo_noalloc.cu",
 ]

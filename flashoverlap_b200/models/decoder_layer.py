@@ -119,6 +119,27 @@ class TPDecoderLayer(nn.Module):
             return out
         return layout.rmsnorm_ref(x, weight, self.cfg.eps)
 
+    @staticmethod
+    def _native(t: torch.Tensor) -> bool:
+        """Whether the fused element-wise kernels take ``t``: 16-bit, contiguous, on a GPU, and no
+        autograd graph to record (they have no backward)."""
+        if not (t.is_cuda and t.dtype in (torch.bfloat16, torch.float16) and t.is_contiguous()
+                and t.data_ptr() % 16 == 0) or (torch.is_grad_enabled() and t.requires_grad):
+            return False
+        from .._build import load
+        load()
+        return True
+
+    def _add_norm(self, x, y, weight):
+        """``(x + y, rmsnorm(x + y) * weight)``."""
+        if (self._native(x) and self._native(y) and x.shape == y.shape and x.dtype == y.dtype == weight.dtype
+                and x.shape[-1] % 8 == 0 and x.shape[-1] <= 16384 and weight.data_ptr() % 16 == 0):
+            h, out = torch.empty_like(x), torch.empty_like(x)
+            torch.ops.flashoverlap_op.add_rmsnorm(x, y, h, out, weight, self.cfg.eps)
+            return h, out
+        h = x + y
+        return h, self._norm(h, weight)
+
     def _all_gather_tokens(self, x_sp: torch.Tensor) -> torch.Tensor:
         if self.world == 1:
             return x_sp
@@ -160,11 +181,16 @@ class TPDecoderLayer(nn.Module):
         if self._gathered:
             # token order for attention; this matrix is (q_local + 2 kv_local) * hd wide, not h
             qkv = layout.gathered_as_tokens(qkv, self.world, TILE_M).reshape(B * S, -1)
+        native_rope = self._native(qkv) and hd % 8 == 0
+        if native_rope:
+            # in place: qkv is this call's own matmul result (or its reordered copy)
+            torch.ops.flashoverlap_op.rope_(qkv, S, self.q_local + self.kv_local, hd, cfg.rope_theta)
         q, k, v = qkv.split([self.q_local * hd, self.kv_local * hd, self.kv_local * hd], dim=-1)
         q = q.view(B, S, self.q_local, hd).transpose(1, 2)
         k = k.view(B, S, self.kv_local, hd).transpose(1, 2)
         v = v.view(B, S, self.kv_local, hd).transpose(1, 2)
-        q, k = _rope(q, cfg.rope_theta), _rope(k, cfg.rope_theta)
+        if not native_rope:
+            q, k = _rope(q, cfg.rope_theta), _rope(k, cfg.rope_theta)
         attn = F.scaled_dot_product_attention(q, k, v, is_causal=True, enable_gqa=True)
         attn = attn.transpose(1, 2).reshape(B * S, self.q_local * hd)
         if self.fuse_norm:
@@ -175,8 +201,8 @@ class TPDecoderLayer(nn.Module):
                                                          cfg.eps, self.algo)
             hn = self._all_gather_tokens(hn_sp)
         else:
-            h_sp = x_sp + self._row_parallel(attn, self.wo)                    # [T/tp, h]
-            hn = self._all_gather_tokens(self._norm(h_sp, self.mlp_norm))
+            h_sp, hn_sp = self._add_norm(x_sp, self._row_parallel(attn, self.wo), self.mlp_norm)   # [T/tp, h]
+            hn = self._all_gather_tokens(hn_sp)
         # MLP block
         gu = torch.matmul(hn, self.wgu.t())
         gate, up = gu.split([self.ffn_local, self.ffn_local], dim=-1)
@@ -189,6 +215,9 @@ class TPDecoderLayer(nn.Module):
         elif self._gathered:
             # out= is closed to autograd: the same placement as a copy of its own
             act = layout.gathered_as_tokens(F.silu(gate) * up, self.world, TILE_M).reshape(B * S, self.ffn_local)
+        elif self._native(gu) and self.ffn_local % 8 == 0:
+            act = torch.empty((B * S, self.ffn_local), dtype=gu.dtype, device=gu.device)
+            torch.ops.flashoverlap_op.swiglu(gu, act)
         else:
             act = F.silu(gate) * up
         return h_sp + self._row_parallel(act, self.wd)

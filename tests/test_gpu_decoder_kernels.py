@@ -1,0 +1,70 @@
+"""Residual add + RMSNorm, rotary embedding and SwiGLU kernels against plain PyTorch."""
+import pytest
+import torch
+import torch.nn.functional as F
+
+from flashoverlap_b200 import ops
+from flashoverlap_b200.models.decoder_layer import _rope
+from flashoverlap_b200.utils import layout
+
+pytestmark = pytest.mark.gpu
+DTYPES = [torch.bfloat16, torch.float16]
+ULP = {torch.bfloat16: 2.0 ** -7, torch.float16: 2.0 ** -10}     # largest spacing of neighbours over the value
+
+
+def _op():
+    return torch.ops.flashoverlap_op
+
+
+# one vector, a remainder in every vectors-per-thread variant, the largest row; one row, several rows per CTA
+@pytest.mark.parametrize("dt", DTYPES)
+@pytest.mark.parametrize("rows,dim", [(1, 8), (3, 2040), (130, 2056), (1500, 4104), (5000, 1024), (33, 8200), (9, 16384)])
+def test_add_rmsnorm(cuda, dt, rows, dim):
+    x, t = torch.randn(rows, dim, device=cuda).to(dt), torch.randn(rows, dim, device=cuda).to(dt)
+    w = (1 + 0.02 * torch.randn(dim, device=cuda)).to(dt)
+    h, y = torch.empty_like(x), torch.empty_like(x)
+    _op().add_rmsnorm(x, t, h, y, w, 1e-5)
+    assert torch.equal(h, x + t)
+    assert torch.equal(y, ops.rmsnorm(h, w, 1e-5))
+    in_place, y2 = x.clone(), torch.empty_like(x)
+    _op().add_rmsnorm(in_place, t, in_place, y2, w, 1e-5)
+    assert torch.equal(in_place, h) and torch.equal(y2, y)
+    ref = layout.rmsnorm_ref(x + t, w, 1e-5).double()
+    assert ((y.double() - ref).abs() <= 2 * ULP[dt] * ref.abs() + 1e-6).all()     # the norm rounds twice
+
+
+def test_add_rmsnorm_refuses(cuda):
+    x = torch.zeros(4, 64, device=cuda, dtype=torch.bfloat16)
+    w = torch.ones(64, device=cuda, dtype=torch.bfloat16)
+    for bad in (x[:, :32], x.half(), x[:2], x.cpu()):
+        with pytest.raises(RuntimeError):
+            _op().add_rmsnorm(x, bad, x.clone(), x.clone(), w, 1e-5)
+
+
+@pytest.mark.parametrize("dt", DTYPES)
+@pytest.mark.parametrize("B,S,heads,extra,hd", [(1, 128, 9, 1, 128), (2, 96, 1, 0, 64), (3, 33, 17, 2, 8), (1, 5000, 8, 8, 128)])
+def test_rope(cuda, dt, B, S, heads, extra, hd):
+    qkv = torch.randn(B * S, (heads + extra) * hd, device=cuda).to(dt)
+    out = qkv.clone()
+    _op().rope_(out, S, heads, hd, 500000.0)
+    got = out[:, :heads * hd].view(B, S, heads, hd).transpose(1, 2)
+    x = qkv[:, :heads * hd].view(B, S, heads, hd).transpose(1, 2)
+    ref = _rope(x, 500000.0)
+    # same angles; a pair's two products may be contracted into one rounding less, so results differ by one
+    # rounding of the result or, where the products cancel, by fp32 roundings of the products
+    mag = x.float().reshape(B, heads, S, hd // 2, 2).norm(dim=-1, keepdim=True).expand(-1, -1, -1, -1, 2).reshape(ref.shape)
+    assert ((got.float() - ref.float()).abs() <= ULP[dt] * ref.float().abs() + 2.0 ** -20 * mag + 2.0 ** -24).all()
+    assert torch.equal(out[:, heads * hd:], qkv[:, heads * hd:])
+
+
+@pytest.mark.parametrize("dt", DTYPES)
+@pytest.mark.parametrize("rows,f", [(1, 8), (7, 2048), (300, 2056), (64, 4104), (5000, 3584)])
+def test_swiglu(cuda, dt, rows, f):
+    gu = (3 * torch.randn(rows, 2 * f, device=cuda)).to(dt)
+    gu[0, 0], gu[0, 1] = -60000.0, float("inf")
+    y = torch.empty(rows, f, device=cuda, dtype=dt)
+    _op().swiglu(gu, y)
+    ref = F.silu(gu[:, :f]) * gu[:, f:]
+    # silu's last fp32 bit may round the 16-bit value the other way, and the product rounds once more
+    same = (y == ref) | ((y - ref).abs() <= 2 * ULP[dt] * ref.abs() + 2.0 ** -19) | (y.isnan() & ref.isnan())
+    assert same.all()
