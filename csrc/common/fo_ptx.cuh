@@ -67,6 +67,15 @@ FO_DEVICE void mbar_arrive_cluster(uint32_t cluster_addr) {
   asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(cluster_addr) : "memory");
 }
 
+// ------------------------------------------------------------------ programmatic dependent launch
+
+// Waits until every grid this one depends on has completed and its writes are visible; returns at
+// once in a grid launched without the programmatic attribute.  Nothing a predecessor may have written,
+// and nothing a predecessor may still read, is touched before it.
+FO_DEVICE void grid_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+// Lets the next grid of the stream start launching (it still waits in grid_wait for this one's end).
+FO_DEVICE void grid_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
 // ------------------------------------------------------------------ mbarrier
 
 FO_DEVICE void mbar_init(uint64_t* bar, uint32_t count) {

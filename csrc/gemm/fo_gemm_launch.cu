@@ -40,7 +40,7 @@ cudaError_t launch_one(const GemmTensorMaps* maps, const GemmParams* p, int grid
   static bool attr_set[16] = {};
   return launch_kernel<CTA2>(fo_gemm_kernel<BN, STAGES, BF16, FUSED, CTA2, MT, A2A, NORM, TRACE, EPI>,
                              FUSED ? kThreadsFused : kThreadsPlain, smem, attr_set, maps, p, grid_x, nvr, cooperative,
-                             stream, query);
+                             false, stream, query);
 }
 
 // One case per kernel of gemm/fo_gemm_instances.inc.

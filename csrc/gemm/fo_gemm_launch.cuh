@@ -8,10 +8,11 @@
 namespace fo {
 
 // Common part of every launch.  query != nullptr: do not launch, report the largest co-resident
-// grid instead.
+// grid instead.  programmatic: the kernel calls ptx::grid_wait before it touches global memory, so
+// its launch and prologue may overlap the tail of the stream's previous kernel.
 template <bool CTA2, typename Kernel, typename Maps>
 cudaError_t launch_kernel(Kernel kernel, int threads, int smem, bool* attr_set, const Maps* maps, const GemmParams* p,
-                          int grid_x, int nvr, bool cooperative, cudaStream_t stream, int* query) {
+                          int grid_x, int nvr, bool cooperative, bool programmatic, cudaStream_t stream, int* query) {
   int dev = 0;
   cudaGetDevice(&dev);
   if (dev >= 0 && dev < 16 && !attr_set[dev]) {
@@ -23,7 +24,7 @@ cudaError_t launch_kernel(Kernel kernel, int threads, int smem, bool* attr_set, 
   cfg.blockDim = dim3(threads, 1, 1);
   cfg.dynamicSmemBytes = smem;
   cfg.stream = stream;
-  cudaLaunchAttribute attr[2];
+  cudaLaunchAttribute attr[3];
   cfg.attrs = attr;
   cfg.numAttrs = 0;
   if (CTA2) {
@@ -54,6 +55,11 @@ cudaError_t launch_kernel(Kernel kernel, int threads, int smem, bool* attr_set, 
   if (cooperative) {
     attr[cfg.numAttrs].id = cudaLaunchAttributeCooperative;
     attr[cfg.numAttrs].val.cooperative = 1;
+    ++cfg.numAttrs;
+  }
+  if (programmatic) {
+    attr[cfg.numAttrs].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[cfg.numAttrs].val.programmaticStreamSerializationAllowed = 1;
     ++cfg.numAttrs;
   }
   return cudaLaunchKernelEx(&cfg, kernel, *maps, *p);

@@ -13,7 +13,7 @@ cudaError_t launch_plain_one(const PlainTensorMaps* maps, const GemmParams* p, i
   static_assert(smem <= 227 * 1024, "shared memory of this configuration exceeds 227 KB");
   static bool attr_set[16] = {};
   return launch_kernel<CTA2>(fo_gemm_plain_kernel<BN, STAGES, BF16, CTA2, MT>, kPlainThreads, smem, attr_set, maps, p,
-                             grid_x, 1, false, stream, query);
+                             grid_x, 1, false, true, stream, query);
 }
 
 template <bool BF16>

@@ -140,6 +140,8 @@ __global__ void __launch_bounds__(kPlainThreads, 1)
   }
   ptx::tc_fence_after_sync();
   const uint32_t tmem_base = *s_tmem_base;
+  ptx::grid_launch_dependents();
+  ptx::grid_wait();
 
   if (warp_idx == 0) {
     // ------------------------------------------------------------------ TMA producer

@@ -19,7 +19,7 @@ cudaError_t launch_one(const SplitTensorMaps& maps, const GemmParams* p, cudaStr
     if (e != cudaSuccess) return e;
     if (dev >= 0 && dev < 16) attr_set[dev] = true;
   }
-  cudaLaunchAttribute attr[1];
+  cudaLaunchAttribute attr[2];
   attr[0].id = cudaLaunchAttributeClusterDimension;
   attr[0].val.clusterDim.x = S;
   attr[0].val.clusterDim.y = 1;
@@ -34,6 +34,9 @@ cudaError_t launch_one(const SplitTensorMaps& maps, const GemmParams* p, cudaStr
     cfg.gridDim = dim3(S, 1, 1);
     return cudaOccupancyMaxActiveClusters(query, kernel, &cfg);
   }
+  attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[1].val.programmaticStreamSerializationAllowed = 1;
+  cfg.numAttrs = 2;
   cfg.gridDim = dim3(p->num_tiles * S, 1, 1);
   return cudaLaunchKernelEx(&cfg, kernel, maps, *p);
 }

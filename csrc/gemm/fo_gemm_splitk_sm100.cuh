@@ -87,6 +87,8 @@ __global__ void __launch_bounds__(kSplitThreads, 1)
   __syncthreads();
   ptx::tc_fence_after_sync();
   const uint32_t tmem_base = *s_tmem_base;
+  ptx::grid_launch_dependents();
+  ptx::grid_wait();
 
   const int ew = warp_idx - 2;
   const int wg = ew >> 2;

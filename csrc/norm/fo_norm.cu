@@ -14,6 +14,8 @@
 #include <cuda_fp16.h>
 #include <cstdint>
 
+#include "../common/fo_ptx.cuh"
+
 namespace fo {
 
 namespace {
@@ -97,6 +99,8 @@ __global__ void __launch_bounds__(kNormThreads, (VPT <= 2 ? 6 : (VPT <= 4 ? 4 : 
   const int per_cta = (rows + gridDim.x - 1) / gridDim.x;
   const int row_begin = blockIdx.x * per_cta;
   const int row_end = min(rows, row_begin + per_cta);
+  ptx::grid_launch_dependents();
+  ptx::grid_wait();
   if (row_begin >= row_end) return;
 
   uint4 wv[VPT];
@@ -192,6 +196,8 @@ __global__ void __launch_bounds__(kNormThreads, (VPT <= 2 ? 4 : 2))
   const int per_cta = (rows + gridDim.x - 1) / gridDim.x;
   const int row_begin = blockIdx.x * per_cta;
   const int row_end = min(rows, row_begin + per_cta);
+  ptx::grid_launch_dependents();
+  ptx::grid_wait();
   if (row_begin >= row_end) return;
   auto load_row = [&](int b, uint4 (&x)[VPT], uint4 (&t)[VPT]) {
     const size_t base = static_cast<size_t>(b) * dim;
@@ -257,6 +263,8 @@ __global__ void __launch_bounds__(kNormThreads, (VPT <= 2 ? 6 : (VPT <= 4 ? 4 : 
   const int per_cta = (rows + gridDim.x - 1) / gridDim.x;
   const int row_begin = blockIdx.x * per_cta;
   const int row_end = min(rows, row_begin + per_cta);
+  ptx::grid_launch_dependents();
+  ptx::grid_wait();
   if (row_begin >= row_end) return;
   const uint4* __restrict__ x = reinterpret_cast<const uint4*>(X);
   uint4* __restrict__ y = reinterpret_cast<uint4*>(Y);
@@ -306,6 +314,37 @@ __global__ void __launch_bounds__(kNormThreads, (VPT <= 2 ? 6 : (VPT <= 4 ? 4 : 
   }
 }
 
+// Launch whose prologue may overlap the tail of the stream's previous kernel (the kernels call
+// ptx::grid_wait before they touch memory): 49.3 -> 45.9 us for a reorder and its inverse over
+// 4096 x 8192, 51.5 -> 50.2 us for the norm of 8192 x 8192.  A CTA that starts while its SM is still set up for a
+// GEMM's 227 KB of shared memory finds 28 KB of L1 for its loads in flight (16384 x 8192 after a GEMM:
+// 328 us the two, 321 us with the carve-out asked for here, 319 us without the early launch).
+template <auto kernel, typename... Args>
+cudaError_t launch_rows(int grid, cudaStream_t stream, Args... args) {
+  // (per kernel and device, and the same whoever sets it)
+  static bool carved[16] = {};
+  int dev = 0;
+  cudaGetDevice(&dev);
+  if (dev >= 0 && dev < 16 && !carved[dev]) {
+    const cudaError_t e =
+        cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxL1);
+    if (e != cudaSuccess) return e;
+    carved[dev] = true;
+  }
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(grid, 1, 1);
+  cfg.blockDim = dim3(kNormThreads, 1, 1);
+  cfg.stream = stream;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  const cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, args...);
+  if (e != cudaSuccess) cudaGetLastError();  // reported to the caller, not left for the next one
+  return e;
+}
+
 // Contiguous row blocks: enough CTAs to fill the machine several times over, yet a few rows per CTA
 // so that the prefetch and the cached tile look-ups pay off.
 int row_grid(int rows, int sm_count) {
@@ -325,17 +364,15 @@ cudaError_t launch_add_norm(const void* X, const void* T, void* H, void* Y, cons
   uint16_t* y = static_cast<uint16_t*>(Y);
   const uint16_t* w = static_cast<const uint16_t*>(W);
   if (vpt <= 1) {
-    add_rmsnorm_kernel<BF16, 1><<<grid, kNormThreads, 0, stream>>>(x, t, h, y, w, rows, dim, eps);
+    return launch_rows<add_rmsnorm_kernel<BF16, 1>>(grid, stream, x, t, h, y, w, rows, dim, eps);
   } else if (vpt <= 2) {
-    add_rmsnorm_kernel<BF16, 2><<<grid, kNormThreads, 0, stream>>>(x, t, h, y, w, rows, dim, eps);
+    return launch_rows<add_rmsnorm_kernel<BF16, 2>>(grid, stream, x, t, h, y, w, rows, dim, eps);
   } else if (vpt <= 4) {
-    add_rmsnorm_kernel<BF16, 4><<<grid, kNormThreads, 0, stream>>>(x, t, h, y, w, rows, dim, eps);
+    return launch_rows<add_rmsnorm_kernel<BF16, 4>>(grid, stream, x, t, h, y, w, rows, dim, eps);
   } else if (vpt <= 8) {
-    add_rmsnorm_kernel<BF16, 8><<<grid, kNormThreads, 0, stream>>>(x, t, h, y, w, rows, dim, eps);
-  } else {
-    return cudaErrorInvalidValue;  // dim > 16384
+    return launch_rows<add_rmsnorm_kernel<BF16, 8>>(grid, stream, x, t, h, y, w, rows, dim, eps);
   }
-  return cudaGetLastError();
+  return cudaErrorInvalidValue;  // dim > 16384
 }
 
 template <bool BF16, bool REORDER>
@@ -348,8 +385,7 @@ cudaError_t launch_norm(const void* X, void* Y, const void* W, int rows, int dim
   uint16_t* y = static_cast<uint16_t*>(Y);
   const uint16_t* w = static_cast<const uint16_t*>(W);
 #define FO_LAUNCH_NORM(V)                                                                      \
-  rmsnorm_kernel<BF16, REORDER, V><<<grid, kNormThreads, 0, stream>>>(x, y, w, rows, dim, BM, BN, \
-                                                                       rldn, RA, eps)
+  return launch_rows<rmsnorm_kernel<BF16, REORDER, V>>(grid, stream, x, y, w, rows, dim, BM, BN, rldn, RA, eps)
   if (vpt <= 1) {
     FO_LAUNCH_NORM(1);
   } else if (vpt <= 2) {
@@ -358,11 +394,9 @@ cudaError_t launch_norm(const void* X, void* Y, const void* W, int rows, int dim
     FO_LAUNCH_NORM(4);
   } else if (vpt <= 8) {
     FO_LAUNCH_NORM(8);
-  } else {
-    return cudaErrorInvalidValue;  // dim > 16384
   }
 #undef FO_LAUNCH_NORM
-  return cudaGetLastError();
+  return cudaErrorInvalidValue;  // dim > 16384
 }
 
 }  // namespace
@@ -406,9 +440,9 @@ cudaError_t reorder_launch(const void* X, void* Y, int rows, int dim, int BM, in
 #define FO_LAUNCH_REORDER(V)                                                                              \
   do {                                                                                                    \
     if (to_reordered) {                                                                                   \
-      reorder_kernel<true, V><<<grid, kNormThreads, 0, stream>>>(x, y, rows, dim, BM, BN, rldn, RA);      \
+      return launch_rows<reorder_kernel<true, V>>(grid, stream, x, y, rows, dim, BM, BN, rldn, RA);           \
     } else {                                                                                              \
-      reorder_kernel<false, V><<<grid, kNormThreads, 0, stream>>>(x, y, rows, dim, BM, BN, rldn, RA);     \
+      return launch_rows<reorder_kernel<false, V>>(grid, stream, x, y, rows, dim, BM, BN, rldn, RA);          \
     }                                                                                                     \
   } while (0)
   if (vpt <= 1) {
@@ -419,11 +453,9 @@ cudaError_t reorder_launch(const void* X, void* Y, int rows, int dim, int BM, in
     FO_LAUNCH_REORDER(4);
   } else if (vpt <= 8) {
     FO_LAUNCH_REORDER(8);
-  } else {
-    return cudaErrorInvalidValue;  // dim > 16384
   }
 #undef FO_LAUNCH_REORDER
-  return cudaGetLastError();
+  return cudaErrorInvalidValue;  // dim > 16384
 }
 
 }  // namespace fo
