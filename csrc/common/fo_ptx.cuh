@@ -45,19 +45,13 @@ FO_DEVICE uint32_t mapa_shared(uint32_t smem_addr, uint32_t rank) {
   asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(smem_addr), "r"(rank));
   return r;
 }
-// Loads from the shared memory of a CTA of this cluster (addresses from mapa_shared).
-FO_DEVICE uint32_t ld_shared_cluster_u32(uint32_t cluster_addr) {
-  uint32_t v;
-  asm volatile("ld.shared::cluster.u32 %0, [%1];" : "=r"(v) : "r"(cluster_addr) : "memory");
-  return v;
+// Stores into the shared memory of a CTA of this cluster (addresses from mapa_shared).
+FO_DEVICE void st_shared_cluster_u32(uint32_t cluster_addr, uint32_t v) {
+  asm volatile("st.shared::cluster.u32 [%0], %1;" ::"r"(cluster_addr), "r"(v) : "memory");
 }
-FO_DEVICE float4 ld_shared_cluster_v4(uint32_t cluster_addr) {
-  float4 v;
-  asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];"
-               : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w)
-               : "r"(cluster_addr)
+FO_DEVICE void st_shared_cluster_v4(uint32_t cluster_addr, uint32_t x, uint32_t y, uint32_t z, uint32_t w) {
+  asm volatile("st.shared::cluster.v4.u32 [%0], {%1, %2, %3, %4};" ::"r"(cluster_addr), "r"(x), "r"(y), "r"(z), "r"(w)
                : "memory");
-  return v;
 }
 // Arrive on an mbarrier that may live in another CTA of the cluster (address from mapa_shared).
 // Release at CTA scope (the instruction's default): what the barrier hands over is TMEM, ordered by

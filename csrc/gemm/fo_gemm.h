@@ -20,6 +20,9 @@ std::string encode_tmap_16bit(CUtensorMap* out, const void* ptr, uint64_t rows, 
 // Fills tiles_m / tiles_n / num_tiles / raster_sw of `p` for `algo` and checks divisibility.
 std::string prepare_tiling(int algo, GemmParams* p);
 
+// Sets p->raster_sw for strips of `strip` N tiles (0: whole row panels) and the tiles in `p`.
+void set_raster(int strip, GemmParams* p);
+
 // Launches the kernel for `algo`.  grid_x CTAs per virtual rank, nvr virtual ranks
 // (gridDim.y).  `cooperative` requests a cooperative launch, which fails instead of
 // deadlocking when the grid cannot be co-resident (needed when CTAs of different virtual
@@ -28,19 +31,20 @@ cudaError_t launch_gemm(int algo, bool bf16, bool fused, const GemmTensorMaps& m
                         const GemmParams& p, int grid_x, int nvr, bool cooperative,
                         cudaStream_t stream);
 
-// Split over K of a GEMM with few tiles (fo_gemm_splitk_sm100.cuh): `split` CTAs of a cluster per
-// 128 x bn tile; split == 0: none.
-struct SplitChoice {
-  int bn, split;
+// What the GEMM without a collective, counters or monitoring runs for `algo`.  A row-major output does
+// not depend on the tiling, a tile-contiguous one only on its tile width p.out_bn, so a small or ragged
+// problem may take another kernel (fewer idle SMs, fewer waves): narrower tiles, CTA pairs (tiles_m may be odd:
+// the last pair's second half is then empty), or the split-K kernel.
+struct PlainPlan {
+  int algo;   // kernel and raster
+  int split;  // 2, 4 or 8: split-K kernel (128 x kSplitBN tiles) instead of algo's
 };
-constexpr int kMinSplitBlocks = 4;  // k-blocks each CTA of a split must have
-// The split for the problem in `p`, tiled 128 x bn.  Splits are for shapes whose tiles all fit the
-// device several times over; a row-major output may be retiled, a tile-contiguous one keeps `bn`.
-// forced: -1 automatic, 0 never, 2 / 4 / 8 that split wherever it fits the device.
-SplitChoice choose_split(const GemmParams& p, int bn, bool bf16, int forced);
-// `b`: tensor map with boxes of c.bn rows; `p`: tile counts of 128 x c.bn tiles.
-cudaError_t launch_splitk_gemm(SplitChoice c, bool bf16, const CUtensorMap& a, const CUtensorMap& b,
-                               const GemmParams& p, cudaStream_t stream);
+constexpr int kSplitBN = 128;
+// split: -1 automatic, 0 never, 2 / 4 / 8 that split wherever it fits the device; exact: algo's own kernel.
+PlainPlan choose_plain(const GemmParams& p, int algo, bool bf16, int split, bool exact);
+// `b`: tensor map with boxes of kSplitBN rows; `p`: tile counts of 128 x kSplitBN tiles.
+cudaError_t launch_splitk_gemm(int split, bool bf16, const CUtensorMap& a, const CUtensorMap& b, const GemmParams& p,
+                               cudaStream_t stream);
 
 // Sets the L2 eviction priorities of the operand loads for the tiling already in `p`: with
 // column strips swept M-major the B strip is re-read by every wave of the strip (keep it: evict

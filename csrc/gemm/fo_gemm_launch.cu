@@ -130,10 +130,13 @@ std::string prepare_tiling(int algo, GemmParams* p) {
   p->tiles_m = p->M / c.bm;
   p->tiles_n = p->N / c.bn;
   p->num_tiles = p->tiles_m * p->tiles_n;
-  int sw = c.raster_sw <= 0 ? p->tiles_n : c.raster_sw;
-  if (sw > p->tiles_n) sw = p->tiles_n;
-  p->raster_sw = sw;
+  p->out_bn = c.bn;
+  set_raster(c.raster_sw, p);
   return "";
+}
+
+void set_raster(int strip, GemmParams* p) {
+  p->raster_sw = strip <= 0 || strip > p->tiles_n ? p->tiles_n : strip;
 }
 
 void set_l2_hints(GemmParams* p, bool enable) {

@@ -46,6 +46,7 @@ struct GemmParams {
   int tiles_m, tiles_n, num_tiles;
   int raster_sw;     // strip width (in N tiles) of the tile sweep
   int out_mode;      // OutMode
+  int out_bn;        // plain kernels: tile width of the tile-contiguous layout (num_tiles counts its tiles)
   int rldn;          // reordered layout: tiles per reordered row (reference rLDN, 1 in practice)
   int signal;        // bump MM[group] after each tile (counter-gated NCCL path)
   int monitor;       // record per-tile completion order in MM rows 1..TM

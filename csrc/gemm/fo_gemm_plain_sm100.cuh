@@ -92,7 +92,9 @@ __global__ void __launch_bounds__(kPlainThreads, 1)
   const int unit = CTA2 ? static_cast<int>(blockIdx.x >> 1) : static_cast<int>(blockIdx.x);
   const int num_units = CTA2 ? static_cast<int>(gridDim.x >> 1) : static_cast<int>(gridDim.x);
   constexpr int kRowsPerUnit = (CTA2 ? 2 : 1) * MT;  // 128-row tiles of one scheduling unit
-  const int sched_tiles_m = p.tiles_m / kRowsPerUnit;
+  // A launch may have fewer row tiles than its units cover (an odd tiles_m under CTA pairs): the TMA
+  // loads of the missing rows return zeros and their tiles are not stored.
+  const int sched_tiles_m = (p.tiles_m + kRowsPerUnit - 1) / kRowsPerUnit;
   const int sched_tiles = sched_tiles_m * p.tiles_n;
   auto my_tile = [&](int pos) {
     TileCoord tc = tile_of_position(pos, sched_tiles_m, p.tiles_n, p.raster_sw);
@@ -296,8 +298,11 @@ __global__ void __launch_bounds__(kPlainThreads, 1)
     for (int pos = unit; pos < sched_tiles; pos += num_units) {
       TileCoord tc = my_tile(pos);
       if constexpr (MT == 2) tc.m += wg;
-      const int t = tc.m * p.tiles_n + tc.n;
-      const int r = tile_position(p, t, status);
+      const bool exists = tc.m < p.tiles_m;
+      // tile of the layout that holds this one: the same, or (out_bn > BN) a wider one
+      const int n0 = tc.n * BN;
+      const int t = tc.m * (p.N / p.out_bn) + n0 / p.out_bn;
+      const int r = exists ? tile_position(p, t, status) : 0;
 
       // Where the tile goes.  TMA stores: coordinates of the warp's first chunk in the output's 2-D
       // view.  Per-thread stores: lane l stores the 16-byte piece (l & 7) of the warp's rows
@@ -305,12 +310,14 @@ __global__ void __launch_bounds__(kPlainThreads, 1)
       int tma_x0 = 0, tma_y0 = 0;
       uint8_t* row_ptr[8];
       uint32_t row_valid = 0xffu;  // bit i clear: row i has no destination
-      if (use_tma) {
+      if (!exists) {
+        row_valid = 0;
+      } else if (use_tma) {
         if (p.out_mode == kOutNatural) {
-          tma_x0 = tc.n * BN;
+          tma_x0 = n0;
           tma_y0 = tc.m * kBM + quad * 32;
-        } else {  // tile-contiguous: [M * N / (rldn * BN)] rows of rldn * BN elements
-          tma_x0 = (r % p.rldn) * BN;
+        } else {  // tile-contiguous: [M * N / (rldn * out_bn)] rows of rldn * out_bn elements
+          tma_x0 = (r % p.rldn) * p.out_bn + n0 % p.out_bn;
           tma_y0 = (r / p.rldn) * kBM + quad * 32;
         }
       } else {
@@ -320,10 +327,11 @@ __global__ void __launch_bounds__(kPlainThreads, 1)
           const int lr = quad * 32 + (lane >> 3) + 4 * i;
           size_t off = 0;  // element offset of (row lr, tile column 0)
           if (p.out_mode == kOutNatural) {
-            off = (static_cast<size_t>(tc.m) * kBM + lr) * p.N + static_cast<size_t>(tc.n) * BN;
+            off = (static_cast<size_t>(tc.m) * kBM + lr) * p.N + n0;
           } else if (p.out_mode == kOutReorder) {
-            const size_t ld = static_cast<size_t>(p.rldn) * BN;
-            off = (static_cast<size_t>(r / p.rldn) * kBM + lr) * ld + static_cast<size_t>(r % p.rldn) * BN;
+            const size_t ld = static_cast<size_t>(p.rldn) * p.out_bn;
+            off = (static_cast<size_t>(r / p.rldn) * kBM + lr) * ld + static_cast<size_t>(r % p.rldn) * p.out_bn +
+                  n0 % p.out_bn;
           } else {  // kOutScatterRows: rows of the [M*N/BN, BN] view are remapped through RE
             const size_t row_id = static_cast<size_t>(r) * kBM + lr;
             const int re = p.RE[row_id];
@@ -368,6 +376,7 @@ __global__ void __launch_bounds__(kPlainThreads, 1)
           __syncwarp();
           if (lane == 0) ptx::mbar_arrive_cluster(tmem_empty_addr0 + static_cast<uint32_t>(acc) * 8u);
         }
+        if (!exists) continue;
         // The buffer is free once the previous store has read it: about 600 cycles after its issue,
         // 900 for a CTA's first store.  On the CTA's last tile nothing hides that and the operand
         // ring is idle (the accumulator is complete, so every load has landed and been multiplied):
@@ -412,7 +421,7 @@ __global__ void __launch_bounds__(kPlainThreads, 1)
         }
       }
 
-      if ((p.signal | p.monitor) != 0 && p.MM[0] != nullptr) {
+      if (exists && (p.signal | p.monitor) != 0 && p.MM[0] != nullptr) {
         // The tile may be announced only once all its stores have been written.
         if (use_tma && lane == 0) {
           ptx::bulk_wait_group<0>();

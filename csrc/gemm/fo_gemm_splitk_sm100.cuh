@@ -2,17 +2,25 @@
 // C = A * B^T written row-major or tile-contiguous, without a collective, counters or monitoring.
 //
 // With one CTA per 128 x BN tile a decode batch (M = 128) or a narrow projection leaves most SMs
-// idle: 128 x 8192 x 3584 is 32 tiles, 32 of 148 SMs, and one SM takes in about 100 GB/s of
-// operands, so reading 59 MB of weights took 23 us.  Here the S CTAs of a cluster share one tile: CTA s
-// multiplies k-blocks [s * kb / S, (s + 1) * kb / S), leaves its fp32 partial sums in its idle
-// operand ring, and after a cluster barrier CTA s adds up the S partials of columns
-// [s * BN / S, (s + 1) * BN / S) through distributed shared memory.  The sums are fp32 and are
+// idle: 128 x 8192 x 3584 is 32 tiles of 128 x 256 on 148 SMs, and one SM takes in 100 - 140 GB/s of
+// operands, so reading 59 MB of weights took 23 us.  Here the S CTAs of a cluster share one 128 x 128
+// tile: CTA s multiplies k-blocks [s * kb / S, (s + 1) * kb / S), sends its fp32 partial sums of the
+// columns that CTA d finishes, [d * 128 / S, (d + 1) * 128 / S), straight from TMEM into d's shared memory,
+// and after a cluster barrier adds up the S partials of its own columns.  The sums are fp32 and are
 // added in the order of the ranks, so results do not depend on timing; no workspace, no second
 // launch.
+//
+// The exchange is what a split costs: distributed shared memory moves about 14 bytes a cycle and SM,
+// so 32 KB (S = 2) take 2,300 cycles and the 96 KB of 128 x 256 tiles split in four took 7,600.  Hence
+// narrow tiles, small splits, a receive buffer of its own (sends need not wait for the receiver's
+// ring) and stores rather than loads.  128 x 8192 x 3584: 25.2 us on 128 x 256 tiles, 16.6 us on 128 x 128
+// tiles, 14.4 us with those split in two (16.5 us in four where that needs two waves of clusters), of
+// which the weights' way through HBM takes 9 us; 128 x 1024 x 28672: 153 us, 19.4 us split in eight.
 //
 // Roles as in fo_gemm_plain_sm100.cuh (warp 0 TMA producer, warp 1 MMA issuer, warps 2-9
 // epilogue); one tile per cluster, so nothing is persistent and TMEM holds one accumulator.
 #pragma once
+#include "fo_gemm.h"
 #include "fo_gemm_device.cuh"
 
 namespace fo {
@@ -23,25 +31,30 @@ struct SplitTensorMaps {
   CUtensorMap a, b;
 };
 
-template <int BN, int STAGES>
+constexpr int kSplitStages = 5;
+
+template <int S>
 struct SplitSmem {
   static constexpr int kABytes = kBM * kBK * 2;
-  static constexpr int kBBytes = BN * kBK * 2;
+  static constexpr int kBBytes = kSplitBN * kBK * 2;
   static constexpr int kStageBytes = kABytes + kBBytes;
-  static constexpr int kBarOffset = STAGES * kStageBytes;
-  static constexpr int kNumBars = 2 * STAGES + 1;
+  // Partial sums from the other CTAs: [S - 1 senders][own columns / 4][128 rows] x 16 bytes;
+  // consecutive lanes (rows) take consecutive vectors.
+  static constexpr int kRecvOffset = kSplitStages * kStageBytes;
+  static constexpr int kOwnCols = kSplitBN / S;
+  static constexpr int kSlotBytes = kOwnCols * kBM * 4;
+  static constexpr int kBarOffset = kRecvOffset + (S - 1) * kSlotBytes;
+  static constexpr int kNumBars = 2 * kSplitStages + 1;
   static constexpr int kMiscOffset = kBarOffset + kNumBars * 8;
-  // Partial sums, [BN / 4][128 rows] x 16 bytes: consecutive lanes (rows) take consecutive vectors.
-  static constexpr int kPartialBytes = BN * kBM * 4;
-  static_assert(kPartialBytes <= kBarOffset, "the ring must hold the partial sums");
   static constexpr int kTotalBytes = kMiscOffset + 16 + 1024;
 };
 
-template <int BN, int STAGES, bool BF16, int S>
+template <bool BF16, int S>
 __global__ void __launch_bounds__(kSplitThreads, 1)
     fo_gemm_splitk_kernel(const __grid_constant__ SplitTensorMaps maps, const __grid_constant__ GemmParams p) {
-  using L = SplitSmem<BN, STAGES>;
-  constexpr int kOwnCols = BN / S;  // columns whose sum this CTA finishes
+  using L = SplitSmem<S>;
+  constexpr int BN = kSplitBN, STAGES = kSplitStages;
+  constexpr int kOwnCols = L::kOwnCols;  // columns whose sum this CTA finishes
   // columns of one warpgroup: half of them, or all (the other idles) when half is below 16
   constexpr int kWgCols = kOwnCols >= 32 ? kOwnCols / 2 : kOwnCols;
   static_assert(kOwnCols % 16 == 0, "columns are summed 16 at a time");
@@ -54,6 +67,7 @@ __global__ void __launch_bounds__(kSplitThreads, 1)
   uint32_t* misc = reinterpret_cast<uint32_t*>(smem + L::kMiscOffset);
   uint32_t* s_tmem_base = misc;
   volatile int* s_abort = reinterpret_cast<volatile int*>(misc + 1);
+  volatile uint32_t* s_peer_failed = misc + 2;  // set by a CTA of the cluster that sent nothing
 
   const int warp_idx = __shfl_sync(0xffffffffu, static_cast<int>(threadIdx.x >> 5), 0);
   const int lane = threadIdx.x & 31;
@@ -73,6 +87,7 @@ __global__ void __launch_bounds__(kSplitThreads, 1)
     }
     ptx::mbar_init(tmem_full_bar, 1);
     *s_abort = 0;
+    *s_peer_failed = 0;
     ptx::mbar_fence_init();
   }
   if (warp_idx == 0 && lane == 0) {
@@ -86,6 +101,9 @@ __global__ void __launch_bounds__(kSplitThreads, 1)
   ptx::tc_fence_before_sync();
   __syncthreads();
   ptx::tc_fence_after_sync();
+  // First phase of the cluster barrier: every CTA runs and has cleared its failure word before
+  // anybody stores into its shared memory.  The epilogue waits for it ahead of its sends.
+  ptx::cluster_arrive_release();
   const uint32_t tmem_base = *s_tmem_base;
   ptx::grid_launch_dependents();
   ptx::grid_wait();
@@ -173,79 +191,81 @@ __global__ void __launch_bounds__(kSplitThreads, 1)
       *s_abort = 1;
     }
     ptx::tc_fence_after_sync();
+    ptx::cluster_wait_acquire();
     if (ok) {
-      // Columns that other CTAs finish go to this CTA's ring: the accumulator is complete, so every
-      // load has landed and been multiplied.
-#pragma unroll 2
+      // Columns that other CTAs finish go to their receive buffers.
+#pragma unroll
       for (int c = wg * 32; c < BN; c += 64) {
         uint32_t v[32];
         ptx::tmem_ld_32x32b_x32(t_row + c, v);
         ptx::tmem_ld_wait();
 #pragma unroll
         for (int h = 0; h < 2; ++h) {
-          if ((c + 16 * h) / kOwnCols == rank) continue;
+          const int c0 = c + 16 * h;
+          const int d = c0 / kOwnCols;  // CTA that finishes these columns
+          if (d == rank) continue;
+          const int slot = rank < d ? rank : rank - 1;
+          const uint32_t dst = ptx::mapa_shared(ptx::smem_u32(smem + L::kRecvOffset), d) +
+                               ((slot * kOwnCols + c0 - d * kOwnCols) / 4 * kBM + row) * 16;
 #pragma unroll
           for (int j = 0; j < 4; ++j) {
             const int b = 16 * h + 4 * j;
-            *reinterpret_cast<uint4*>(smem + (((c + b) / 4) * kBM + row) * 16) =
-                make_uint4(v[b], v[b + 1], v[b + 2], v[b + 3]);
+            ptx::st_shared_cluster_v4(dst + j * kBM * 16, v[b], v[b + 1], v[b + 2], v[b + 3]);
           }
         }
       }
+    } else if (lane < S) {
+      ptx::st_shared_cluster_u32(ptx::mapa_shared(ptx::smem_u32(misc + 2), lane), 1u);
     }
   }
+  if (warp_idx < 2) ptx::cluster_wait_acquire();
 
-  // Every CTA's partial sums are written (release / acquire at cluster scope).
+  // Every CTA's partial sums have arrived (release / acquire at cluster scope).
   ptx::cluster_arrive_release();
   ptx::cluster_wait_acquire();
 
   if (warp_idx >= 2) {
     // ------------------------------------------------------------------ epilogue, second half
-    size_t off;  // element offset of (this row, tile column 0)
-    if (p.out_mode == kOutNatural) {
-      off = (static_cast<size_t>(tc.m) * kBM + row) * p.N + static_cast<size_t>(tc.n) * BN;
-    } else {
-      const int r = tile_position(p, tc.m * p.tiles_n + tc.n, status);
-      const size_t ld = static_cast<size_t>(p.rldn) * BN;
-      off = (static_cast<size_t>(r / p.rldn) * kBM + row) * ld + static_cast<size_t>(r % p.rldn) * BN;
-    }
-    // a CTA that gave up left no partial sums: nobody in the cluster stores (the status says why)
-    uint32_t gave_up = 0;
-#pragma unroll
-    for (int s = 0; s < S; ++s) {
-      gave_up |= ptx::ld_shared_cluster_u32(ptx::mapa_shared(ptx::smem_u32(misc + 1), s));
-    }
-    if (gave_up == 0 && (kOwnCols >= 32 || wg == 0)) {
-      uint32_t peer[S];
-#pragma unroll
-      for (int s = 0; s < S; ++s) peer[s] = ptx::mapa_shared(ptx::smem_u32(smem), s);
+    // (A CTA that gave up sent nothing: nobody in the cluster stores, the status says why.)
+    if (*s_peer_failed == 0 && (kOwnCols >= 32 || wg == 0)) {
+      const int n0 = tc.n * BN;
+      size_t off;  // element offset of (this row, tile column 0)
+      if (p.out_mode == kOutNatural) {
+        off = (static_cast<size_t>(tc.m) * kBM + row) * p.N + n0;
+      } else {
+        const int r = tile_position(p, tc.m * (p.N / p.out_bn) + n0 / p.out_bn, status);
+        const size_t ld = static_cast<size_t>(p.rldn) * p.out_bn;
+        off = (static_cast<size_t>(r / p.rldn) * kBM + row) * ld + static_cast<size_t>(r % p.rldn) * p.out_bn +
+              n0 % p.out_bn;
+      }
       uint8_t* out = reinterpret_cast<uint8_t*>(p.out[0]);
-#pragma unroll 1
+#pragma unroll
       for (int i = 0; i < kWgCols; i += 16) {
-        const int c = rank * kOwnCols + (kOwnCols >= 32 ? wg * kWgCols : 0) + i;
+        const int oc = (kOwnCols >= 32 ? wg * kWgCols : 0) + i;  // among the own columns
+        const int c = rank * kOwnCols + oc;                      // in the tile
         uint32_t own[16];
         ptx::tmem_ld_32x32b_x16(t_row + c, own);
-        float4 x[S][4];
-#pragma unroll
-        for (int s = 0; s < S; ++s) {
-#pragma unroll
-          for (int j = 0; j < 4; ++j) {
-            if (s != rank) x[s][j] = ptx::ld_shared_cluster_v4(peer[s] + ((c / 4 + j) * kBM + row) * 16);
-          }
-        }
         ptx::tmem_ld_wait();
         float a[16];
 #pragma unroll
         for (int j = 0; j < 16; ++j) a[j] = 0.f;
 #pragma unroll
         for (int s = 0; s < S; ++s) {
+          const int slot = s < rank ? s : s - 1;
 #pragma unroll
           for (int j = 0; j < 4; ++j) {
-            const bool mine = s == rank;
-            a[4 * j + 0] += mine ? __uint_as_float(own[4 * j + 0]) : x[s][j].x;
-            a[4 * j + 1] += mine ? __uint_as_float(own[4 * j + 1]) : x[s][j].y;
-            a[4 * j + 2] += mine ? __uint_as_float(own[4 * j + 2]) : x[s][j].z;
-            a[4 * j + 3] += mine ? __uint_as_float(own[4 * j + 3]) : x[s][j].w;
+            float4 x;
+            if (s == rank) {
+              x = make_float4(__uint_as_float(own[4 * j]), __uint_as_float(own[4 * j + 1]),
+                              __uint_as_float(own[4 * j + 2]), __uint_as_float(own[4 * j + 3]));
+            } else {
+              x = *reinterpret_cast<const float4*>(smem + L::kRecvOffset +
+                                                   (((slot * kOwnCols + oc) / 4 + j) * kBM + row) * 16);
+            }
+            a[4 * j + 0] += x.x;
+            a[4 * j + 1] += x.y;
+            a[4 * j + 2] += x.z;
+            a[4 * j + 3] += x.w;
           }
         }
 #pragma unroll
@@ -261,10 +281,9 @@ __global__ void __launch_bounds__(kSplitThreads, 1)
     }
   }
 
+  // Nobody stores into another CTA's shared memory after the barrier: each leaves by itself.
   ptx::tc_fence_before_sync();
-  // Nobody leaves while another CTA of the cluster may still read its partial sums.
-  ptx::cluster_arrive_relaxed();
-  ptx::cluster_wait_acquire();
+  __syncthreads();
   if (warp_idx == 1) {
     ptx::tc_fence_after_sync();
     ptx::tmem_dealloc(tmem_base, BN);

@@ -98,17 +98,17 @@ inline void setup_stage_map(GemmTensorMaps* maps, int rank, void* stage, const G
 }
 
 // Output map of a plain kernel for virtual rank `vr`: the row-major [M, N] output, or the
-// tile-contiguous layout viewed as [M * N / (rldn * BN), rldn * BN], box 32 x 64 (one epilogue
+// tile-contiguous layout viewed as [M * N / (rldn * out_bn), rldn * out_bn], box 32 x 64 (one epilogue
 // warp's chunk).  Sets p->tma_out when the layout can be described that way; otherwise the kernel keeps its
 // per-thread stores (row-scatter and all-to-all outputs, a tile count that rldn does not divide,
 // an output whose address is not 16-byte aligned).
-inline void setup_out_map(GemmTensorMaps* maps, int vr, void* out, GemmParams* p, int bn) {
+inline void setup_out_map(GemmTensorMaps* maps, int vr, void* out, GemmParams* p) {
   if (vr == 0) p->tma_out = 0;
   uint64_t cols = 0;
   if (p->out_mode == kOutNatural) {
     cols = static_cast<uint64_t>(p->N);
   } else if (p->out_mode == kOutReorder && p->rldn >= 1 && p->num_tiles % p->rldn == 0) {
-    cols = static_cast<uint64_t>(p->rldn) * bn;
+    cols = static_cast<uint64_t>(p->rldn) * p->out_bn;
   } else {
     return;
   }

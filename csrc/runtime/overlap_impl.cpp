@@ -116,6 +116,8 @@ void OverlapImpl::SetOption(std::string name, int64_t value) {
   } else if (name == "tma_out") {
     FO_CHECK(value >= -1 && value <= 1, "tma_out must be -1 (automatic), 0 or 1");
     opt_tma_out_ = value;
+  } else if (name == "exact_algo") {
+    opt_exact_algo_ = value ? 1 : 0;
   } else if (name == "split_k") {
     FO_CHECK(value == -1 || value == 0 || value == 2 || value == 4 || value == 8,
              "split_k must be -1 (automatic), 0 (never), 2, 4 or 8");
@@ -139,6 +141,7 @@ int64_t OverlapImpl::GetOption(std::string name) {
   if (name == "stage_local") return opt_stage_local_;
   if (name == "epi_bufs") return opt_epi_bufs_;
   if (name == "tma_out") return opt_tma_out_;
+  if (name == "exact_algo") return opt_exact_algo_;
   if (name == "split_k") return opt_split_k_;
   if (name == "validate") return opt_validate_;
   if (name == "wait_sleep_ns") return opt_wait_sleep_ns_;
@@ -288,7 +291,6 @@ void OverlapImpl::run_plain(const at::Tensor& A, const at::Tensor& B, void* out,
   std::memset(&p, 0, sizeof(p));
   bool bf16 = true;
   setup_problem(algo, A, B, 0, &maps, &p, &bf16);
-  set_l2_hints(&p, opt_l2_hints_ != 0);
   p.out_mode = out_mode;
   p.rldn = rldn < 1 ? 1 : rldn;
   p.signal = signal ? 1 : 0;
@@ -306,24 +308,33 @@ void OverlapImpl::run_plain(const at::Tensor& A, const at::Tensor& B, void* out,
   p.out[0] = out;
   p.MM[0] = MM;
   p.status[0] = status_.data_ptr<int>();
-  const SplitChoice split = choose_split(p, algo_config(algo).bn, bf16, static_cast<int>(opt_split_k_));
-  if (split.split != 0) {
-    p.tiles_n = p.N / split.bn;
-    p.num_tiles = p.tiles_m * p.tiles_n;
-    if (p.raster_sw > p.tiles_n) p.raster_sw = p.tiles_n;
-    const std::string e = encode_tmap_16bit(&maps.b[0], B.data_ptr(), p.N, p.K, split.bn);
+  const PlainPlan plan =
+      choose_plain(p, algo, bf16, static_cast<int>(opt_split_k_), opt_exact_algo_ != 0);
+  const AlgoConfig c = algo_config(plan.algo);
+  const int bn = plan.split != 0 ? kSplitBN : c.bn;
+  const int b_rows = plan.split == 0 && c.cta2 ? bn / 2 : bn;
+  const AlgoConfig own = algo_config(algo);
+  if (b_rows != (own.cta2 ? own.bn / 2 : own.bn)) {
+    const std::string e = encode_tmap_16bit(&maps.b[0], B.data_ptr(), p.N, p.K, b_rows);
     FO_CHECK(e.empty(), "B: ", e);
-    cuda_check(launch_splitk_gemm(split, bf16, maps.a[0], maps.b[0], p, stream()), "split-K GEMM launch");
+  }
+  p.tiles_n = p.N / bn;
+  set_raster(c.raster_sw, &p);
+  set_l2_hints(&p, opt_l2_hints_ != 0);
+  if (plan.split != 0) {
+    cuda_check(launch_splitk_gemm(plan.split, bf16, maps.a[0], maps.b[0], p, stream()), "split-K GEMM launch");
     return;
   }
   // TMA tensor stores wherever the output can be described as a 2-D tensor: never slower than the
   // per-thread stores (1024 x 4096 x 1024: 15.3 against 15.6 us for the 256 x 256-per-CTA kernel,
   // 10.0 against 9.9 us for the 128 x 256 one).
   const bool tma_out = opt_tma_out_ != 0;
-  if (tma_out) setup_out_map(&maps, 0, out, &p, algo_config(algo).bn);
-  const int resident = gemm_max_resident_ctas(algo, bf16, false);
-  const int grid = std::max(1, std::min(std::min(grid_cap, resident), p.num_tiles));
-  cuda_check(launch_gemm(algo, bf16, false, maps, p, grid, 1, false, stream()), "GEMM launch");
+  if (tma_out) setup_out_map(&maps, 0, out, &p);
+  const int resident = gemm_max_resident_ctas(plan.algo, bf16, false);
+  const int pair = c.cta2 ? 2 : 1;
+  const int ctas = (p.tiles_m + pair - 1) / pair * pair * p.tiles_n;
+  const int grid = std::max(1, std::min(std::min(grid_cap, resident), ctas));
+  cuda_check(launch_gemm(plan.algo, bf16, false, maps, p, grid, 1, false, stream()), "GEMM launch");
 }
 
 void OverlapImpl::Gemm(at::Tensor A, at::Tensor B, at::Tensor C, int64_t Algo) {

@@ -195,6 +195,7 @@ class OverlapImpl : public torch::CustomClassHolder {
 #else
   int64_t opt_validate_ = 0;     // 1: also check the VALUES of RA / RE / cSEG_GPU (a device-to-host copy per call)
 #endif
+  int64_t opt_exact_algo_ = 0;   // plain GEMM: 1 runs the Algo's own kernel even where another is faster
   int64_t opt_split_k_ = -1;     // plain GEMM of few tiles split over K: -1 automatic, 0 never, else that many CTAs a tile
   int64_t opt_tma_out_ = -1;     // plain kernels' stores: 0 per-thread stores, else TMA tensor stores where the output allows
   int64_t opt_pull_direct_ = -1;  // pull protocol: epilogue threads store the partials themselves (1), TMA (0), by kernel (-1)

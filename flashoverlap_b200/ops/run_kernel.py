@@ -63,6 +63,7 @@ def main() -> None:
             impl = ops.OverlapImpl()
             impl.nccl_init(0, 1, [0] * 16)
             impl.cutlass_init()
+            impl.set_option("exact_algo", 1)           # time the kernel each Algo names, not a faster stand-in
             if a.kernel == "gemm":
                 fn = lambda: impl.cutlass_gemm(A, B, C, a.algo)
             else:

@@ -68,3 +68,32 @@ def test_split_gemm_reordered(cuda, impl, M, N, K, algo, rldn):
     finally:
         impl.set_option("split_k", -1)
     impl.check_status()
+
+
+# odd row tiles on pairs, 512-row units with nothing to fill them, 256-wide tiles computed as 128-wide ones
+@pytest.mark.parametrize("M,N,K,algo", [(1920, 5376, 1000, 0), (512, 4096, 520, 3), (256, 8192, 320, 1), (640, 1152, 200, 2)])
+def test_stand_in_kernels(cuda, impl, M, N, K, algo):
+    """A small or ragged problem may run on another kernel than its Algo's: same values, same layout."""
+    dt = torch.bfloat16
+    a = (torch.randn(M, K, device=cuda) * 0.5).to(dt)
+    b = (torch.randn(N, K, device=cuda) * 0.5).to(dt)
+    p = config.algo_params(algo)
+    tm, tn = M // p["BM"], N // p["BN"]
+    RA = torch.randperm(tm * tn, device=cuda, dtype=torch.int32)
+    rldn = 2 if tm * tn % 2 == 0 else 1
+    e = torch.empty(0, dtype=torch.int32)
+    mm = torch.zeros(tm + 1, tn, device=cuda, dtype=torch.int32)
+    try:
+        for exact, tma in ((1, -1), (0, -1), (0, 0)):
+            impl.set_option("exact_algo", exact)
+            impl.set_option("tma_out", tma)
+            c = torch.full((M, N), float("nan"), device=cuda, dtype=dt)
+            impl.cutlass_gemm(a, b, c, algo)
+            _check(c, a, b, dt)
+            c.fill_(float("nan"))
+            impl.gemm_allreduce_overlap(a, b, c, mm, RA, rldn, e, e.to(cuda), algo, False)
+            _check(layout.from_reordered(c.cpu(), M, N, p["BM"], p["BN"], RA.cpu(), rldn).to(cuda), a, b, dt)
+    finally:
+        impl.set_option("exact_algo", 0)
+        impl.set_option("tma_out", -1)
+    impl.check_status()

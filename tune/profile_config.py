@@ -29,6 +29,7 @@ def main():
     impl = ops.OverlapImpl()
     impl.nccl_init(0, 1, [0] * 16)
     impl.cutlass_init()
+    impl.set_option("exact_algo", 1)           # time the kernel each Algo names, not a faster stand-in
     A, B = make_operands(args.m, args.n, args.k, dt, "cuda")
     C = torch.empty(args.m, args.n, device="cuda", dtype=dt)
     timed = []
