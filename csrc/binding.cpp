@@ -253,6 +253,8 @@ TORCH_LIBRARY(flashoverlap_class, m) {
       .def("gemm_all2all_fused", &OverlapImpl::GemmAll2AllFused)
       .def("gemm_reducescatter_rmsnorm_fused", &OverlapImpl::GemmReduceScatterRmsNormFused)
       .def("gemm_reducescatter_add_rmsnorm_fused", &OverlapImpl::GemmReduceScatterAddRmsNormFused)
+      .def("gemm_add", &OverlapImpl::GemmAdd)
+      .def("gemm_swiglu", &OverlapImpl::GemmSwiGLU)
       .def("set_option", &OverlapImpl::SetOption)
       .def("get_option", &OverlapImpl::GetOption)
       .def("symm_empty", &OverlapImpl::SymmEmpty)

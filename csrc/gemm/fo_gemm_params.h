@@ -21,6 +21,13 @@ enum OutMode : int {
   kOutAll2All = 3,      // row m goes to the rank and row that a2a_tab assigns to it (all-to-all kernels)
 };
 
+// What the epilogue of the plain kernels does with the fp32 accumulators before it stores them.
+enum PlainEpilogue : int {
+  kEpiStore = 0,     // C = round16(A B^T)
+  kEpiResidual = 1,  // C = round16(round16(A B^T) + R), R row-major like C, which it may be
+  kEpiSwiGLU = 2,    // C = round16(silu(A G^T) * (A U^T)), B = [G; U]: C has half of B's rows as columns
+};
+
 enum CommMode : int {
   kCommNone = 0,
   kCommFusedAR = 2,
@@ -118,6 +125,8 @@ struct GemmParams {
   // (row-major [M, N], or the tile-contiguous layout as [M * N / (rldn * BN), rldn * BN]) and
   // finished chunks leave shared memory as TMA tensor stores; 0 = per-thread 16-byte stores.
   int tma_out;
+  int epilogue;     // plain kernels: PlainEpilogue
+  const void* res;  // kEpiResidual: row-major [M, N]
   // Back-off of the roles that wait on mbarriers with slack (TMA producer, MMA issuer, push warp;
   // four times as long for the epilogue's wait for its accumulator): nanoseconds slept between
   // polls once a wait has turned out to be a long one.  0 = poll continuously.

@@ -62,11 +62,23 @@ struct PlainSmem {
   static constexpr int kTotalBytes = kMiscOffset + 16 + 1024;
 };
 
-template <int BN, int STAGES, bool BF16, bool CTA2, int MT>
+template <bool BF16>
+__device__ __forceinline__ uint4 add8(const uint4& a, const uint4& b) {
+  return make_uint4(add2<BF16>(a.x, b.x), add2<BF16>(a.y, b.y), add2<BF16>(a.z, b.z), add2<BF16>(a.w, b.w));
+}
+
+__device__ __forceinline__ float silu_mul(uint32_t g, uint32_t u) {
+  const float x = __uint_as_float(g);
+  return x / (1.f + expf(-x)) * __uint_as_float(u);
+}
+
+template <int BN, int STAGES, bool BF16, bool CTA2, int MT, int EPI>
 __global__ void __launch_bounds__(kPlainThreads, 1)
     fo_gemm_plain_kernel(const __grid_constant__ PlainTensorMaps maps, const __grid_constant__ GemmParams p) {
   static_assert(MT == 1 || (MT == 2 && CTA2 && BN == 256), "two row halves need CTA pairs and BN = 256");
+  static_assert(EPI != kEpiSwiGLU || (CTA2 && MT == 1 && BN == 256), "the two CTAs of a pair load the two halves of B");
   using L = PlainSmem<BN, STAGES, CTA2, MT>;
+  constexpr int kOutCols = EPI == kEpiSwiGLU ? BN / 2 : BN;  // output columns of a tile
   // Accumulator slots in TMEM: two tiles in flight (MT = 1) or the two halves of one (MT = 2).
   constexpr int kAccStages = MT == 2 ? 1 : 2;
   extern __shared__ uint8_t smem_raw[];
@@ -172,8 +184,11 @@ __global__ void __launch_bounds__(kPlainThreads, 1)
               ptx::tma_load_2d_pair(sa + h * L::kAHalfBytes, &maps.a, &full_bar[stage], kb * kBK, (tc.m + h) * kBM,
                                     p.l2_hint_a);
             }
-            ptx::tma_load_2d_pair(sb, &maps.b, &full_bar[stage], kb * kBK,
-                                  tc.n * BN + static_cast<int>(cta_rank) * L::kBRows, p.l2_hint_b);
+            // SwiGLU: the leader loads 128 rows of G, the follower the same rows of U, and so the tile's
+            // accumulators hold the 128 gate columns and then the 128 up columns.
+            const int b_row = EPI == kEpiSwiGLU ? static_cast<int>(cta_rank) * p.N + tc.n * kOutCols
+                                                : tc.n * BN + static_cast<int>(cta_rank) * L::kBRows;
+            ptx::tma_load_2d_pair(sb, &maps.b, &full_bar[stage], kb * kBK, b_row, p.l2_hint_b);
           } else {
             ptx::mbar_arrive_expect_tx(&full_bar[stage], L::kStageBytes);
             ptx::tma_load_2d(sa, &maps.a, &full_bar[stage], kb * kBK, tc.m * kBM, p.l2_hint_a);
@@ -300,7 +315,7 @@ __global__ void __launch_bounds__(kPlainThreads, 1)
       if constexpr (MT == 2) tc.m += wg;
       const bool exists = tc.m < p.tiles_m;
       // tile of the layout that holds this one: the same, or (out_bn > BN) a wider one
-      const int n0 = tc.n * BN;
+      const int n0 = tc.n * kOutCols;
       const int t = tc.m * (p.N / p.out_bn) + n0 / p.out_bn;
       const int r = exists ? tile_position(p, t, status) : 0;
 
@@ -347,6 +362,19 @@ __global__ void __launch_bounds__(kPlainThreads, 1)
         }
       }
 
+      // Residual: the warp's 32 rows x 64 columns of a chunk, a chunk ahead, 8 lanes to a row.
+      [[maybe_unused]] uint4 res[8];
+      [[maybe_unused]] auto load_residual = [&](int c) {
+        const uint8_t* src = reinterpret_cast<const uint8_t*>(p.res) +
+                             ((static_cast<size_t>(tc.m) * kBM + quad * 32 + (lane >> 3)) * p.N + n0 + c * 64) * 2 +
+                             (lane & 7) * 16;
+#pragma unroll
+        for (int i = 0; i < 8; ++i) res[i] = ptx::ld_cg_v4(src + static_cast<size_t>(4 * i) * p.N * 2);
+      };
+      if constexpr (EPI == kEpiResidual) {
+        if (exists) load_residual(MT == 2 ? 0 : wg);
+      }
+
       // A warp that gives up goes on through the loop without touching data: the others may be
       // waiting for it at the tile barrier below.
       if (ok) {
@@ -362,15 +390,27 @@ __global__ void __launch_bounds__(kPlainThreads, 1)
       const uint32_t t_row = tmem_base + (static_cast<uint32_t>(quad * 32) << 16) +
                              static_cast<uint32_t>((MT == 2 ? wg : acc) * BN);
       constexpr int kChunkStep = MT == 2 ? 1 : 2;
-      static_assert(kPlainEpilogueWarps * (BN / 64) * L::kWarpBufBytes <= L::kEpiOffset, "the ring must hold a tile");
+      static_assert(kPlainEpilogueWarps * (kOutCols / 64) * L::kWarpBufBytes <= L::kEpiOffset, "the ring must hold a tile");
       const bool last_tile = pos + num_units >= sched_tiles;
 #pragma unroll 1
-      for (int c = MT == 2 ? 0 : wg; ok && c < BN / 64; c += kChunkStep) {
+      for (int c = MT == 2 ? 0 : wg; ok && c < kOutCols / 64; c += kChunkStep) {
         uint32_t v0[32], v1[32];
         ptx::tmem_ld_32x32b_x32(t_row + c * 64, v0);
         ptx::tmem_ld_32x32b_x32(t_row + c * 64 + 32, v1);
-        ptx::tmem_ld_wait();
-        if (c + kChunkStep >= BN / 64) {
+        if constexpr (EPI == kEpiSwiGLU) {
+          uint32_t u0[32], u1[32];
+          ptx::tmem_ld_32x32b_x32(t_row + kOutCols + c * 64, u0);
+          ptx::tmem_ld_32x32b_x32(t_row + kOutCols + c * 64 + 32, u1);
+          ptx::tmem_ld_wait();
+#pragma unroll
+          for (int i = 0; i < 32; ++i) {
+            v0[i] = __float_as_uint(silu_mul(v0[i], u0[i]));
+            v1[i] = __float_as_uint(silu_mul(v1[i], u1[i]));
+          }
+        } else {
+          ptx::tmem_ld_wait();
+        }
+        if (c + kChunkStep >= kOutCols / 64) {
           // Accumulator fully read by this warp: hand it back to the (leader's) MMA warp.
           ptx::tc_fence_before_sync();
           __syncwarp();
@@ -384,11 +424,21 @@ __global__ void __launch_bounds__(kPlainThreads, 1)
         uint8_t* cbuf = buf;
         if (use_tma) {
           if (last_tile && c >= kChunkStep) {
-            cbuf = smem + (ew * (BN / 64) + c) * L::kWarpBufBytes;
+            cbuf = smem + (ew * (kOutCols / 64) + c) * L::kWarpBufBytes;
           } else {
             if (lane == 0) ptx::bulk_wait_group_read<0>();
             __syncwarp();
           }
+        }
+        if constexpr (EPI == kEpiResidual) {
+          // to the layout of the accumulators (a row per lane), through the buffer
+#pragma unroll
+          for (int i = 0; i < 8; ++i) {
+            const int lr = (lane >> 3) + 4 * i;
+            *reinterpret_cast<uint4*>(cbuf + lr * 128 + (((lane & 7) ^ (lr & 7)) * 16)) = res[i];
+          }
+          __syncwarp();
+          if (c + kChunkStep < kOutCols / 64) load_residual(c + kChunkStep);
         }
         // Row `lane` of the warp's slice, 16-byte pieces swizzled as the tensor store expects.
 #pragma unroll
@@ -400,7 +450,9 @@ __global__ void __launch_bounds__(kPlainThreads, 1)
           w.y = pack2<BF16>(__uint_as_float(v[b + 2]), __uint_as_float(v[b + 3]));
           w.z = pack2<BF16>(__uint_as_float(v[b + 4]), __uint_as_float(v[b + 5]));
           w.w = pack2<BF16>(__uint_as_float(v[b + 6]), __uint_as_float(v[b + 7]));
-          *reinterpret_cast<uint4*>(cbuf + lane * 128 + ((j ^ (lane & 7)) * 16)) = w;
+          uint4* piece = reinterpret_cast<uint4*>(cbuf + lane * 128 + ((j ^ (lane & 7)) * 16));
+          if constexpr (EPI == kEpiResidual) w = add8<BF16>(w, *piece);
+          *piece = w;
         }
         if (use_tma) {
           ptx::fence_proxy_async_smem();  // generic-proxy writes before the async-proxy read

@@ -275,6 +275,10 @@ __global__ void __launch_bounds__(kSplitThreads, 1)
           w.y = pack2<BF16>(a[8 * h + 2], a[8 * h + 3]);
           w.z = pack2<BF16>(a[8 * h + 4], a[8 * h + 5]);
           w.w = pack2<BF16>(a[8 * h + 6], a[8 * h + 7]);
+          if (p.res != nullptr) {  // residual, laid out like the row-major output (which it may be)
+            const uint4 r = ptx::ld_cg_v4(reinterpret_cast<const uint8_t*>(p.res) + (off + c + 8 * h) * 2);
+            w = make_uint4(add2<BF16>(w.x, r.x), add2<BF16>(w.y, r.y), add2<BF16>(w.z, r.z), add2<BF16>(w.w, r.w));
+          }
           ptx::st_v4(out + (off + c + 8 * h) * 2, w);
         }
       }

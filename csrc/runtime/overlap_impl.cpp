@@ -283,7 +283,7 @@ void OverlapImpl::Resync() {
 void OverlapImpl::run_plain(const at::Tensor& A, const at::Tensor& B, void* out, int out_mode,
                             const int* RA, const int* RE, int rldn, int* MM, int mm_stride,
                             bool signal, bool monitor, const int* cseg, int num_groups, int algo,
-                            int grid_cap) {
+                            int grid_cap, const void* res) {
   if (heap_ == nullptr) NcclInit(0, 1, {});
   c10::cuda::CUDAGuard guard(A.device());
   GemmTensorMaps maps;
@@ -308,6 +308,8 @@ void OverlapImpl::run_plain(const at::Tensor& A, const at::Tensor& B, void* out,
   p.out[0] = out;
   p.MM[0] = MM;
   p.status[0] = status_.data_ptr<int>();
+  p.epilogue = res != nullptr ? kEpiResidual : kEpiStore;
+  p.res = res;
   const PlainPlan plan =
       choose_plain(p, algo, bf16, static_cast<int>(opt_split_k_), opt_exact_algo_ != 0);
   const AlgoConfig c = algo_config(plan.algo);
@@ -343,6 +345,58 @@ void OverlapImpl::Gemm(at::Tensor A, at::Tensor B, at::Tensor C, int64_t Algo) {
   check_out(C, A, static_cast<int64_t>(s.M) * s.N, "C");
   run_plain(A, B, C.data_ptr(), kOutNatural, nullptr, nullptr, 1, nullptr, 0, false, false, nullptr,
             0, static_cast<int>(Algo), sm_count_);
+}
+
+void OverlapImpl::GemmAdd(at::Tensor A, at::Tensor B, at::Tensor R, at::Tensor C, int64_t Algo) {
+  NvtxRange nvtx_range("flashoverlap::gemm_add");
+  const GemmShape s = check_operands(A, B);
+  check_out(C, A, static_cast<int64_t>(s.M) * s.N, "C");
+  check_out(R, A, static_cast<int64_t>(s.M) * s.N, "R");
+  FO_CHECK(reinterpret_cast<uintptr_t>(R.data_ptr()) % 16 == 0, "R must be 16-byte aligned");
+  run_plain(A, B, C.data_ptr(), kOutNatural, nullptr, nullptr, 1, nullptr, 0, false, false, nullptr,
+            0, static_cast<int>(Algo), sm_count_, R.data_ptr());
+}
+
+void OverlapImpl::GemmSwiGLU(at::Tensor A, at::Tensor B, at::Tensor C) {
+  NvtxRange nvtx_range("flashoverlap::gemm_swiglu");
+  if (heap_ == nullptr) NcclInit(0, 1, {});
+  c10::cuda::CUDAGuard guard(A.device());
+  const GemmShape s = check_operands(A, B);
+  const int f = s.N / 2;
+  FO_CHECK(s.M % kBM == 0 && s.N % 256 == 0 && s.K % 8 == 0, "gemm_swiglu needs M a multiple of 128, ",
+           "B of 2 * N rows with N a multiple of 128, and K a multiple of 8 (M=", s.M, " rows of B=", s.N, " K=", s.K, ")");
+  check_out(C, A, static_cast<int64_t>(s.M) * f, "C");
+  constexpr int kPairAlgo = 1;  // CTA pairs, 256-wide B tiles, strips of 8
+  GemmTensorMaps maps;
+  GemmParams p;
+  std::memset(&p, 0, sizeof(p));
+  p.M = s.M;
+  p.N = f;
+  p.K = s.K;
+  p.tiles_m = s.M / kBM;
+  p.tiles_n = f / 128;
+  p.num_tiles = p.tiles_m * p.tiles_n;
+  p.out_bn = 128;
+  p.out_mode = kOutNatural;
+  p.rldn = 1;
+  p.comm = kCommNone;
+  p.ws = 1;
+  p.epilogue = kEpiSwiGLU;
+  p.timeout_ns = static_cast<uint64_t>(opt_timeout_ms_) * 1000000ull;
+  p.wait_sleep_ns = static_cast<uint32_t>(opt_wait_sleep_ns_);
+  p.out[0] = C.data_ptr();
+  p.status[0] = status_.data_ptr<int>();
+  set_raster(algo_config(kPairAlgo).raster_sw, &p);
+  set_l2_hints(&p, opt_l2_hints_ != 0);
+  std::string e = encode_tmap_16bit(&maps.a[0], A.data_ptr(), s.M, s.K, kBM);
+  FO_CHECK(e.empty(), "A: ", e);
+  e = encode_tmap_16bit(&maps.b[0], B.data_ptr(), s.N, s.K, 128);
+  FO_CHECK(e.empty(), "B: ", e);
+  setup_out_map(&maps, 0, C.data_ptr(), &p);
+  FO_CHECK(p.tma_out != 0, "C must be 16-byte aligned");
+  const int resident = gemm_max_resident_ctas(kPairAlgo, s.bf16, false);
+  const int grid = std::max(2, std::min(resident, (p.tiles_m + 1) / 2 * 2 * p.tiles_n));
+  cuda_check(launch_gemm(kPairAlgo, s.bf16, false, maps, p, grid, 1, false, stream()), "SwiGLU GEMM launch");
 }
 
 // ---------------------------------------------------------------------------- bare collectives
@@ -636,18 +690,17 @@ void OverlapImpl::GemmReduceScatterAddRmsNormFused(at::Tensor A, at::Tensor B, a
   NvtxRange nvtx_range("flashoverlap::gemm_reducescatter_add_rmsnorm_fused");
   FO_CHECK(heap_ != nullptr, "call nccl_init first");
   if (world_ == 1) {
-    // One rank: nothing to reduce; GEMM, then residual add and RMSNorm in one pass over the rows.
+    // One rank: nothing to reduce; GEMM that adds the residual, then the stand-alone RMSNorm.
     const GemmShape s = check_operands(A, B);
     FO_CHECK(W.is_cuda() && W.is_contiguous() && W.scalar_type() == A.scalar_type() && W.numel() == s.N,
              "W must be a contiguous CUDA tensor of N elements in the operands' dtype");
     check_out(R, A, static_cast<int64_t>(s.M) * s.N, "R");
     check_out(Y, A, static_cast<int64_t>(s.M) * s.N, "Y");
-    at::Tensor tmp = at::empty({s.M, s.N}, A.options());
-    Gemm(A, B, tmp, Algo);
     at::Tensor r2 = R.view({s.M, s.N});
-    cuda_check(add_rmsnorm_launch(r2.data_ptr(), tmp.data_ptr(), r2.data_ptr(), Y.data_ptr(), W.data_ptr(), s.M, s.N,
-                                  static_cast<float>(eps), s.bf16, sm_count_, stream()),
-               "add_rmsnorm");
+    GemmAdd(A, B, r2, r2, Algo);
+    cuda_check(rmsnorm_launch(r2.data_ptr(), Y.data_ptr(), W.data_ptr(), s.M, s.N, static_cast<float>(eps), s.bf16,
+                              sm_count_, stream()),
+               "rmsnorm");
     return;
   }
   run_fused(kCommFusedRS, A, B, R, kOutNatural, nullptr, 1, nullptr, 0, false, nullptr, 0,

@@ -66,6 +66,11 @@ class OverlapImpl : public torch::CustomClassHolder {
   // i.e. what follows a sequence-parallel o_proj or down_proj, in the kernel that computes it.
   void GemmReduceScatterAddRmsNormFused(at::Tensor A, at::Tensor B, at::Tensor R, at::Tensor Y, at::Tensor W,
                                         double eps, int64_t Algo);
+  // Single-rank GEMMs with what follows them in a transformer block done in the epilogue:
+  //   C <- A * B^T + R        (R row-major like C; C may be R)
+  //   C <- silu(A * G^T) * (A * U^T)   B = [G; U], G and U [N, K] each, C [M, N]
+  void GemmAdd(at::Tensor A, at::Tensor B, at::Tensor R, at::Tensor C, int64_t Algo);
+  void GemmSwiGLU(at::Tensor A, at::Tensor B, at::Tensor C);
   // GEMM whose epilogue stores every row of A * B^T straight into the receive buffer D of the
   // rank it is bound for, over NVLink; same row bookkeeping as gemm_all2all (mLen_CPU[r][i]
   // rows go from rank r to rank i, runs packed in rank order, own run excluded), no C and no
@@ -142,7 +147,8 @@ class OverlapImpl : public torch::CustomClassHolder {
   struct FusedArgs;
   void run_plain(const at::Tensor& A, const at::Tensor& B, void* out, int out_mode,
                  const int* RA, const int* RE, int rldn, int* MM, int mm_stride, bool signal,
-                 bool monitor, const int* cseg, int num_groups, int algo, int grid_cap);
+                 bool monitor, const int* cseg, int num_groups, int algo, int grid_cap,
+                 const void* res = nullptr);
   void run_fused(int comm, const at::Tensor& A, const at::Tensor& B, at::Tensor out, int out_mode,
                  const int* RA, int rldn, int* MM, int mm_stride, bool monitor, const int* cseg,
                  int num_groups, int algo, const at::Tensor* norm_w = nullptr, double norm_eps = 0.0,

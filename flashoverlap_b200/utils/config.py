@@ -155,22 +155,24 @@ def load_tuned(M: int, N: int, K: int, tp: Optional[int] = None, comm_op: Option
     return cfg
 
 
-def default_solution(M: int, N: int, algo: int = 0, wave_size: int = 148, groups: Optional[List[int]] = None) -> dict:
-    """A usable config without any tuning run: analytic hint and one wave per group."""
-    from . import layout
-    p = algo_params(algo)
-
+def fitting_algo(M: int, N: int, algo: int = 0) -> int:
+    """``algo`` where its tile divides the shape, else the Algo of the same raster with the nearest kernel
+    that does (CTA pairs, then one CTA per 128 x 256 tile, then BN = 128); ``algo`` if none does."""
     def fits(k):
         bn, _, cta2, mt = _KERNELS[k]
         return N % bn == 0 and M % ((2 if cta2 else 1) * mt * BM) == 0
 
-    if not fits(p["kernel"]):
-        # nearest kernel that divides the shape: CTA pairs, then one CTA per 128 x 256 tile, then BN = 128
-        for k in (1, 0, 2):
-            if fits(k):
-                algo = algo_with_kernel(algo, k)
-                p = algo_params(algo)
-                break
+    for k in (algo_kernel(algo), 1, 0, 2):
+        if fits(k):
+            return algo_with_kernel(algo, k)
+    return algo
+
+
+def default_solution(M: int, N: int, algo: int = 0, wave_size: int = 148, groups: Optional[List[int]] = None) -> dict:
+    """A usable config without any tuning run: analytic hint and one wave per group."""
+    from . import layout
+    algo = fitting_algo(M, N, algo)
+    p = algo_params(algo)
     tiles = (M // p["BM"]) * (N // p["BN"])
     hint = layout.analytic_hint(M, N, p["BM"], p["BN"], p["raster"], p["rows_per_unit"])
     nw = layout.div_up(tiles, wave_size)

@@ -68,3 +68,49 @@ def test_swiglu(cuda, dt, rows, f):
     # silu's last fp32 bit may round the 16-bit value the other way, and the product rounds once more
     same = (y == ref) | ((y - ref).abs() <= 2 * ULP[dt] * ref.abs() + 2.0 ** -19) | (y.isnan() & ref.isnan())
     assert same.all()
+
+
+@pytest.fixture(scope="module")
+def impl(cuda):
+    i = ops.OverlapImpl()
+    i.nccl_init(0, 1, [0] * 16)
+    i.cutlass_init()
+    return i
+
+
+# a split over K, one wave of pairs, an odd number of row tiles, N that only 128-wide tiles divide, 512-row units
+@pytest.mark.parametrize("dt", DTYPES)
+@pytest.mark.parametrize("M,N,K,algo", [(128, 1024, 512, 0), (256, 2048, 1000, 1), (640, 5376, 264, 0), (384, 1152, 128, 2),
+                                        (1024, 8192, 192, 3)])
+def test_gemm_add(cuda, impl, dt, M, N, K, algo):
+    a, b = torch.randn(M, K, device=cuda).to(dt), (0.1 * torch.randn(N, K, device=cuda)).to(dt)
+    r = torch.randn(M, N, device=cuda).to(dt)
+    for tma, exact in ((-1, 0), (0, 0), (-1, 1)):
+        impl.set_option("tma_out", tma)
+        impl.set_option("exact_algo", exact)
+        plain, out = torch.empty_like(r), torch.empty_like(r)
+        impl.cutlass_gemm(a, b, plain, algo)
+        impl.gemm_add(a, b, r, out, algo)
+        assert torch.equal(out, r + plain)
+        in_place = r.clone()
+        impl.gemm_add(a, b, in_place, in_place, algo)
+        assert torch.equal(in_place, out)
+    impl.set_option("tma_out", -1)
+    impl.set_option("exact_algo", 0)
+    impl.check_status()
+
+
+@pytest.mark.parametrize("dt", DTYPES)
+@pytest.mark.parametrize("M,F_,K", [(128, 128, 64), (256, 1152, 1000), (640, 3584, 264), (4096, 2048, 512)])
+def test_gemm_swiglu(cuda, impl, dt, M, F_, K):
+    a, w = torch.randn(M, K, device=cuda).to(dt), (0.1 * torch.randn(2 * F_, K, device=cuda)).to(dt)
+    out = torch.full((M, F_), float("nan"), device=cuda, dtype=dt)
+    impl.gemm_swiglu(a, w, out)
+    impl.check_status()
+    gu = a.double() @ w.double().t()
+    g, u = gu[:, :F_], gu[:, F_:]
+    ref = F.silu(g) * u
+    # fp32 sums: relative 2^-18 of the magnitudes that were added; silu's slope is below 1.1
+    mag = a.double().abs() @ w.double().abs().t()
+    bound = 0.51 * ULP[dt] * ref.abs() + 2.0 ** -18 * (1.1 * mag[:, :F_] * u.abs() + F.silu(g).abs() * mag[:, F_:]) + 2.0 ** -24
+    assert ((out.double() - ref).abs() <= bound).all()
