@@ -12,6 +12,7 @@
 
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
+#include <algorithm>
 #include <cstdint>
 
 #include "../common/fo_ptx.cuh"
@@ -85,12 +86,15 @@ __device__ __forceinline__ size_t reordered_offset(int b, int col, int dim, int 
 }
 
 // Each CTA takes a contiguous block of rows; each thread owns VPT 16-byte vectors of a row
-// (VPT * 256 * 8 >= dim).  Two things keep HBM busy: the next row's vectors are requested
-// before the current row is reduced (register double buffer), and in the reordered case the
-// tile look-up through RA - a dependent load in front of every data load - is done only when
-// the block of rows crosses into another row panel, not per row.
+// (VPT * 256 * 8 >= dim).  Bound by memory.  Row-major input: the next row's vectors are requested
+// before the current row is reduced (register double buffer).  Tile-contiguous input: a CTA's first
+// loads wait for the look-ups of its tiles through RA, which more CTAs per SM hide better than a
+// row of prefetch in each (six of 40 registers a thread instead of four of 64); the look-up is done
+// only when the block of rows crosses into another row panel, not per row.  16384 x 8192 in tiles of
+// 64 x 256: 93.4 -> 88.6 us, 4096 x 4096: 17.9 -> 14.6 us, 8192 x 16384: 106.8 -> 98.7 us.
 template <bool BF16, bool REORDER, int VPT>
-__global__ void __launch_bounds__(kNormThreads, (VPT <= 2 ? 6 : (VPT <= 4 ? 4 : 2)))
+__global__ void __launch_bounds__(kNormThreads, REORDER ? (VPT <= 2 ? 8 : (VPT <= 4 ? 6 : 3))
+                                                        : (VPT <= 2 ? 6 : (VPT <= 4 ? 4 : 2)))
     rmsnorm_kernel(const uint16_t* __restrict__ X, uint16_t* __restrict__ Y,
                    const uint16_t* __restrict__ W, int rows, int dim, int BM, int BN, int rldn,
                    const int* __restrict__ RA, float eps) {
@@ -103,11 +107,14 @@ __global__ void __launch_bounds__(kNormThreads, (VPT <= 2 ? 6 : (VPT <= 4 ? 4 : 
   ptx::grid_wait();
   if (row_begin >= row_end) return;
 
-  uint4 wv[VPT];
+  // Row-major input: the weights stay in registers.  Tile-contiguous: re-read from L1 per row.
+  [[maybe_unused]] uint4 wv[VPT];
+  if constexpr (!REORDER) {
 #pragma unroll
-  for (int i = 0; i < VPT; ++i) {
-    const int j = threadIdx.x + i * kNormThreads;
-    if (j < nvec) wv[i] = *reinterpret_cast<const uint4*>(W + static_cast<size_t>(j) * 8);
+    for (int i = 0; i < VPT; ++i) {
+      const int j = threadIdx.x + i * kNormThreads;
+      if (j < nvec) wv[i] = *reinterpret_cast<const uint4*>(W + static_cast<size_t>(j) * 8);
+    }
   }
 
   // Offset, in 16-byte vectors, of (row 0 of the current panel, this thread's column) per vector;
@@ -144,10 +151,15 @@ __global__ void __launch_bounds__(kNormThreads, (VPT <= 2 ? 6 : (VPT <= 4 ? 4 : 
     }
   };
 
-  uint4 cur[VPT], nxt[VPT];
-  load_row(row_begin, cur);
+  uint4 cur[VPT];
+  [[maybe_unused]] uint4 nxt[VPT];
+  if constexpr (!REORDER) load_row(row_begin, cur);
   for (int b = row_begin; b < row_end; ++b) {
-    if (b + 1 < row_end) load_row(b + 1, nxt);
+    if constexpr (REORDER) {
+      load_row(b, cur);
+    } else {
+      if (b + 1 < row_end) load_row(b + 1, nxt);
+    }
     float ss = 0.f;
 #pragma unroll
     for (int i = 0; i < VPT; ++i) {
@@ -167,16 +179,24 @@ __global__ void __launch_bounds__(kNormThreads, (VPT <= 2 ? 6 : (VPT <= 4 ? 4 : 
     for (int i = 0; i < VPT; ++i) {
       const int j = threadIdx.x + i * kNormThreads;
       if (j < nvec) {
+        uint4 w;
+        if constexpr (REORDER) {
+          w = __ldg(reinterpret_cast<const uint4*>(W + static_cast<size_t>(j) * 8));
+        } else {
+          w = wv[i];
+        }
         uint4 y;
-        y.x = scale_mul2<BF16>(cur[i].x, wv[i].x, scale);
-        y.y = scale_mul2<BF16>(cur[i].y, wv[i].y, scale);
-        y.z = scale_mul2<BF16>(cur[i].z, wv[i].z, scale);
-        y.w = scale_mul2<BF16>(cur[i].w, wv[i].w, scale);
+        y.x = scale_mul2<BF16>(cur[i].x, w.x, scale);
+        y.y = scale_mul2<BF16>(cur[i].y, w.y, scale);
+        y.z = scale_mul2<BF16>(cur[i].z, w.z, scale);
+        y.w = scale_mul2<BF16>(cur[i].w, w.w, scale);
         __stcs(reinterpret_cast<uint4*>(Y + static_cast<size_t>(b) * dim + static_cast<size_t>(j) * 8), y);
       }
     }
+    if constexpr (!REORDER) {
 #pragma unroll
-    for (int i = 0; i < VPT; ++i) cur[i] = nxt[i];
+      for (int i = 0; i < VPT; ++i) cur[i] = nxt[i];
+    }
   }
 }
 
@@ -353,6 +373,9 @@ int row_grid(int rows, int sm_count) {
   return grid < 1 ? 1 : grid;
 }
 
+// The same with `per` rows per CTA (down to one while that leaves the machine short of CTAs).
+int row_grid(int rows, int sm_count, int per) { return rows <= sm_count * 8 ? rows : (rows + per - 1) / per; }
+
 template <bool BF16>
 cudaError_t launch_add_norm(const void* X, const void* T, void* H, void* Y, const void* W, int rows, int dim,
                             float eps, int sm_count, cudaStream_t stream) {
@@ -380,7 +403,17 @@ cudaError_t launch_norm(const void* X, void* Y, const void* W, int rows, int dim
                         int rldn, const int* RA, float eps, int sm_count, cudaStream_t stream) {
   const int nvec = dim / 8;
   const int vpt = (nvec + kNormThreads - 1) / kNormThreads;
-  const int grid = row_grid(rows, sm_count);
+  // Measured (us, rows per CTA -> time).  Row-major, 8192 x 8192: 2 -> 42.9, 4 -> 45.9, 8 -> 47.6, and the
+  // same order at 4096 x 4096 and 8192 x 16384; rows of up to 2048 elements want more (16384 x 2048:
+  // 2 -> 29.3, 7 -> 27.6).  Tile-contiguous: 8192 x 8192 2 -> 49.0, 4 -> 49.4, 8 -> 55.8; 4096 x 8192 2 -> 28.0,
+  // 4 -> 30.6; 16384 x 2048 4 -> 35.4, 8 -> 34.0; 16384 x 512 4 -> 25.3, 16 -> 23.1.
+  int grid = row_grid(rows, sm_count);
+  if (REORDER) {
+    const int per = vpt > 2 ? std::min(4, rows / 2048) : std::min(vpt == 2 ? 8 : 16, rows / 1024);
+    grid = row_grid(rows, sm_count, std::max(1, per));
+  } else if (vpt > 1) {
+    grid = row_grid(rows, sm_count, 2);
+  }
   const uint16_t* x = static_cast<const uint16_t*>(X);
   uint16_t* y = static_cast<uint16_t*>(Y);
   const uint16_t* w = static_cast<const uint16_t*>(W);
@@ -434,7 +467,9 @@ cudaError_t reorder_launch(const void* X, void* Y, int rows, int dim, int BM, in
   if (rows == 0) return cudaSuccess;
   const int nvec = dim / 8;
   const int vpt = (nvec + kNormThreads - 1) / kNormThreads;
-  const int grid = row_grid(rows, sm_count);
+  // Two rows (what a thread has in flight) per CTA, four where rows are narrow or fill the registers:
+  // 16384 x 8192 2 -> 83.5 us, 4 -> 84.9, 7 -> 89.1; 16384 x 512 2 -> 15.6, 4 -> 13.2; 8192 x 16384 2 -> 106, 4 -> 93.4.
+  const int grid = row_grid(rows, sm_count, vpt == 1 || vpt > 4 ? 4 : 2);
   const uint16_t* x = static_cast<const uint16_t*>(X);
   uint16_t* y = static_cast<uint16_t*>(Y);
 #define FO_LAUNCH_REORDER(V)                                                                              \
