@@ -65,7 +65,7 @@ struct GemmParams {
   int strided_rows;  // 1: row i of a tile belongs to rank i % ws (reference), 0: contiguous
   int diag;          // diagnostic switches (timing studies only): 1 skip the reduction's memory
                      // traffic, 2 skip the push stores, 4 skip the reducers' flag waits
-  int push_lag;      // tiles whose pushes may be in flight before their arrival is signalled (1..4)
+  int push_lag;      // tiles whose pushes may be in flight before their arrival is signalled (1..4; 0: none)
   uint32_t epoch_done_prev;  // value `done` must have reached before the first push
   uint32_t epoch_done;       // value `done` reaches when this call is complete everywhere
   uint64_t timeout_ns;       // bound for every cross-GPU wait

@@ -959,8 +959,8 @@ __global__ void __launch_bounds__(FUSED ? kThreadsFused : kThreadsPlain, 1)
         const int rows_owned = kBM / p.ws;
         const uint8_t* epi = smem + L::kEpiOffset;
         // Tiles of stores kept in flight before the oldest one's completion is awaited.  Stores
-        // into the local staging (pull protocol) complete within a microsecond or two: no lag.
-        const int lag = p.stage_local ? 0 : (p.push_lag < 1 ? 1 : (p.push_lag > kMaxLag ? kMaxLag : p.push_lag));
+        // that stay on this GPU (pull protocol, emulated ranks) complete within a microsecond or two: no lag.
+        const int lag = p.stage_local || p.push_lag < 1 ? 0 : (p.push_lag > kMaxLag ? kMaxLag : p.push_lag);
         int ring[kMaxLag];       // wave groups of the tiles whose pushes may still be in flight
         int ring_t[kMaxLag];     // their tile ids
         int ring_head = 0, ring_count = 0;
