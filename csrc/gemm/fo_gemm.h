@@ -39,6 +39,17 @@ struct PlainPlan {
   int algo;   // kernel and raster
   int split;  // 2, 4 or 8: split-K kernel (128 x kSplitBN tiles) instead of algo's
 };
+// Scheduling units (CTAs, pairs) of a plain kernel's tiles.
+inline int plain_units(const GemmParams& p, int algo) {
+  const AlgoConfig c = algo_config(algo);
+  const int rows = (c.cta2 ? 2 : 1) * c.mt;  // 128-row tiles of a unit
+  return (p.tiles_m + rows - 1) / rows * (p.N / c.bn);
+}
+// Units of the last wave that are computed as halves: all of them if their halves fit one wave.
+inline int plain_tail(int units, int slots) {
+  const int tail = units % slots;
+  return 2 * tail <= slots ? tail : 0;
+}
 constexpr int kSplitBN = 128;
 // split: -1 automatic, 0 never, 2 / 4 / 8 that split wherever it fits the device; exact: algo's own kernel.
 PlainPlan choose_plain(const GemmParams& p, int algo, bool bf16, int split, bool exact);

@@ -40,7 +40,7 @@ enum CommMode : int {
 // launch, each rank with its own operands.
 struct GemmTensorMaps {
   CUtensorMap a[kMaxVirtualRanks];
-  CUtensorMap b[kMaxVirtualRanks];
+  CUtensorMap b[kMaxVirtualRanks];  // plain kernels: b[1] is b[0] with boxes of half the rows (tail_start)
   // fused kernels: every rank's staging buffer viewed as [ws * tiles * rows_owned, BN], box
   // (rows_owned x 64): the epilogue's pushes are TMA stores through these.  Pull variant: this
   // rank's own staging viewed as [tiles * 128, BN], box (128 x 64).  Plain kernels: st[0] is
@@ -125,6 +125,9 @@ struct GemmParams {
   // (row-major [M, N], or the tile-contiguous layout as [M * N / (rldn * BN), rldn * BN]) and
   // finished chunks leave shared memory as TMA tensor stores; 0 = per-thread 16-byte stores.
   int tma_out;
+  // Plain kernels with CTA pairs on 256 x 256 tiles: scheduling positions from here on are computed as two
+  // 256 x 128 halves (the number of positions: none).
+  int tail_start;
   int epilogue;     // plain kernels: PlainEpilogue
   const void* res;  // kEpiResidual: row-major [M, N]
   // Back-off of the roles that wait on mbarriers with slack (TMA producer, MMA issuer, push warp;

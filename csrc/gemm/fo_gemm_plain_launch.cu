@@ -58,6 +58,7 @@ cudaError_t launch_plain_gemm(int kidx, bool bf16, const GemmTensorMaps* maps, c
     pm.a = maps->a[0];
     pm.b = maps->b[0];
     pm.st = maps->st[0];
+    pm.b_half = maps->b[1];
   }
   switch (p != nullptr ? p->epilogue : kEpiStore) {
     case kEpiStore:

@@ -30,6 +30,11 @@
 // 11.5 -> 10.2 us; 256 x 256 per CTA, whose epilogue is exposed at every tile: 17.4 -> 15.3 us, and
 // 229 -> 200 us at 16384 x 8192 x 1024.
 //
+// Last wave.  With CTA pairs on 256 x 256 tiles the tiles left over after the last full wave are computed
+// as 256 x 128 halves when those fit one wave (tail_start): the wave then takes 0.64 of a full one.
+// 1920 x 5376 x 1000 (168 units on 74 pairs): 26.2 -> 24.2 us; projection + residual + norm of
+// 2048 x 8192 x 1792 (256 units): 76.7 -> 75.1 us a call.
+//
 // Every wait is bounded: on expiry the role records a status code, raises a CTA-wide abort
 // flag, the producer drains its TMA loads in flight, TMEM is freed and the kernel returns.
 #pragma once
@@ -44,6 +49,7 @@ constexpr int kPlainThreads = 64 + 32 * kPlainEpilogueWarps;
 // tensor (GemmParams::tma_out), box 32 x 64.
 struct PlainTensorMaps {
   CUtensorMap a, b, st;
+  CUtensorMap b_half;  // half-width tiles of the last wave (GemmParams::tail_start): boxes of half of b's rows
 };
 
 template <int BN, int STAGES, bool CTA2 = false, int MT = 1>
@@ -108,10 +114,22 @@ __global__ void __launch_bounds__(kPlainThreads, 1)
   // loads of the missing rows return zeros and their tiles are not stored.
   const int sched_tiles_m = (p.tiles_m + kRowsPerUnit - 1) / kRowsPerUnit;
   const int sched_tiles = sched_tiles_m * p.tiles_n;
-  auto my_tile = [&](int pos) {
-    TileCoord tc = tile_of_position(pos, sched_tiles_m, p.tiles_n, p.raster_sw);
-    tc.m = kRowsPerUnit * tc.m + MT * static_cast<int>(cta_rank);  // first half; halves follow
-    return tc;
+  // Positions from tail_start on are two half-width tiles each, side by side in the schedule.
+  constexpr bool kHalves = CTA2 && MT == 1 && BN == 256 && EPI != kEpiSwiGLU;
+  const int sched_len = kHalves ? 2 * sched_tiles - p.tail_start : sched_tiles;
+  struct Work {
+    TileCoord tc;
+    bool narrow;  // BN / 2 columns from n0
+    int n0;       // first output column
+  };
+  auto my_tile = [&](int i) {
+    Work w;
+    w.narrow = kHalves && i >= p.tail_start;
+    const int pos = w.narrow ? p.tail_start + (i - p.tail_start) / 2 : i;
+    w.tc = tile_of_position(pos, sched_tiles_m, p.tiles_n, p.raster_sw);
+    w.tc.m = kRowsPerUnit * w.tc.m + MT * static_cast<int>(cta_rank);  // first half; halves follow
+    w.n0 = w.tc.n * kOutCols + (w.narrow ? ((i - p.tail_start) & 1) * (BN / 2) : 0);
+    return w;
   };
   int32_t* status = p.status[0];
   const uint64_t pipe_timeout = 4ull * p.timeout_ns + 1000000000ull;
@@ -164,8 +182,9 @@ __global__ void __launch_bounds__(kPlainThreads, 1)
     uint32_t phase = 0;
     uint32_t issued = 0;
     bool ok = true;
-    for (int pos = unit; ok && pos < sched_tiles; pos += num_units) {
-      const TileCoord tc = my_tile(pos);
+    for (int pos = unit; ok && pos < sched_len; pos += num_units) {
+      const Work work = my_tile(pos);
+      const TileCoord tc = work.tc;
       for (int kb = 0; kb < num_kb; ++kb) {
         if (!ptx::mbar_wait_bounded(&empty_bar[stage], phase ^ 1u, s_abort, pipe_timeout, p.wait_sleep_ns)) {
           if (elected) ptx::report_status(status, kStatusTimeoutSmemEmpty, pos, kb, stage);
@@ -178,7 +197,10 @@ __global__ void __launch_bounds__(kPlainThreads, 1)
         if (elected) {
           if constexpr (CTA2) {
             // The leader's barrier collects the bytes of both CTAs.
-            if (leader) ptx::mbar_arrive_expect_tx(&full_bar[stage], 2 * L::kStageBytes);
+            if (leader) {
+              ptx::mbar_arrive_expect_tx(&full_bar[stage],
+                                         2 * (work.narrow ? L::kStageBytes - L::kBBytes / 2 : L::kStageBytes));
+            }
 #pragma unroll
             for (int h = 0; h < MT; ++h) {
               ptx::tma_load_2d_pair(sa + h * L::kAHalfBytes, &maps.a, &full_bar[stage], kb * kBK, (tc.m + h) * kBM,
@@ -186,9 +208,14 @@ __global__ void __launch_bounds__(kPlainThreads, 1)
             }
             // SwiGLU: the leader loads 128 rows of G, the follower the same rows of U, and so the tile's
             // accumulators hold the 128 gate columns and then the 128 up columns.
-            const int b_row = EPI == kEpiSwiGLU ? static_cast<int>(cta_rank) * p.N + tc.n * kOutCols
-                                                : tc.n * BN + static_cast<int>(cta_rank) * L::kBRows;
-            ptx::tma_load_2d_pair(sb, &maps.b, &full_bar[stage], kb * kBK, b_row, p.l2_hint_b);
+            const int rank = static_cast<int>(cta_rank);
+            if (kHalves && work.narrow) {
+              ptx::tma_load_2d_pair(sb, &maps.b_half, &full_bar[stage], kb * kBK, work.n0 + rank * (L::kBRows / 2),
+                                    p.l2_hint_b);
+            } else {
+              const int b_row = EPI == kEpiSwiGLU ? rank * p.N + work.n0 : work.n0 + rank * L::kBRows;
+              ptx::tma_load_2d_pair(sb, &maps.b, &full_bar[stage], kb * kBK, b_row, p.l2_hint_b);
+            }
           } else {
             ptx::mbar_arrive_expect_tx(&full_bar[stage], L::kStageBytes);
             ptx::tma_load_2d(sa, &maps.a, &full_bar[stage], kb * kBK, tc.m * kBM, p.l2_hint_a);
@@ -220,13 +247,14 @@ __global__ void __launch_bounds__(kPlainThreads, 1)
     // ------------------------------------------------------------------ MMA issuer
     if (leader) {
       const bool elected = ptx::elect_one();
-      constexpr uint32_t idesc = ptx::make_idesc_f16(BF16, CTA2 ? 2 * kBM : kBM, BN);
+      constexpr uint32_t idesc_full = ptx::make_idesc_f16(BF16, CTA2 ? 2 * kBM : kBM, BN);
+      constexpr uint32_t idesc_half = ptx::make_idesc_f16(BF16, CTA2 ? 2 * kBM : kBM, BN / 2);
       int stage = 0;
       uint32_t phase = 0;
       int acc = 0;
       uint32_t acc_phase = 0;
       bool ok = true;
-      for (int pos = unit; ok && pos < sched_tiles; pos += num_units) {
+      for (int pos = unit; ok && pos < sched_len; pos += num_units) {
         if (!ptx::mbar_wait_bounded(&tmem_empty_bar[acc], acc_phase ^ 1u, s_abort, pipe_timeout, p.wait_sleep_ns)) {
           if (elected) ptx::report_status(status, kStatusTimeoutTmemEmpty, pos, acc, 0);
           *s_abort = 1;
@@ -234,6 +262,7 @@ __global__ void __launch_bounds__(kPlainThreads, 1)
         }
         ptx::tc_fence_after_sync();
         const uint32_t tmem_d = tmem_base + static_cast<uint32_t>(acc * BN);
+        const uint32_t idesc = kHalves && pos >= p.tail_start ? idesc_half : idesc_full;
         for (int kb = 0; kb < num_kb; ++kb) {
           if (!ptx::mbar_wait_bounded(&full_bar[stage], phase, s_abort, pipe_timeout, p.wait_sleep_ns)) {
             if (elected) ptx::report_status(status, kStatusTimeoutSmemFull, pos, kb, stage);
@@ -310,12 +339,14 @@ __global__ void __launch_bounds__(kPlainThreads, 1)
     const uint32_t tmem_empty_addr0 =
         CTA2 ? ptx::mapa_shared(ptx::smem_u32(&tmem_empty_bar[0]), 0u) : ptx::smem_u32(&tmem_empty_bar[0]);
 
-    for (int pos = unit; pos < sched_tiles; pos += num_units) {
-      TileCoord tc = my_tile(pos);
+    for (int pos = unit; pos < sched_len; pos += num_units) {
+      const Work work = my_tile(pos);
+      TileCoord tc = work.tc;
       if constexpr (MT == 2) tc.m += wg;
       const bool exists = tc.m < p.tiles_m;
       // tile of the layout that holds this one: the same, or (out_bn > BN) a wider one
-      const int n0 = tc.n * kOutCols;
+      const int n0 = work.n0;
+      const int chunks = (kHalves && work.narrow ? BN / 2 : kOutCols) / 64;
       const int t = tc.m * (p.N / p.out_bn) + n0 / p.out_bn;
       const int r = exists ? tile_position(p, t, status) : 0;
 
@@ -391,9 +422,9 @@ __global__ void __launch_bounds__(kPlainThreads, 1)
                              static_cast<uint32_t>((MT == 2 ? wg : acc) * BN);
       constexpr int kChunkStep = MT == 2 ? 1 : 2;
       static_assert(kPlainEpilogueWarps * (kOutCols / 64) * L::kWarpBufBytes <= L::kEpiOffset, "the ring must hold a tile");
-      const bool last_tile = pos + num_units >= sched_tiles;
+      const bool last_tile = pos + num_units >= sched_len;
 #pragma unroll 1
-      for (int c = MT == 2 ? 0 : wg; ok && c < kOutCols / 64; c += kChunkStep) {
+      for (int c = MT == 2 ? 0 : wg; ok && c < chunks; c += kChunkStep) {
         uint32_t v0[32], v1[32];
         ptx::tmem_ld_32x32b_x32(t_row + c * 64, v0);
         ptx::tmem_ld_32x32b_x32(t_row + c * 64 + 32, v1);
@@ -410,7 +441,7 @@ __global__ void __launch_bounds__(kPlainThreads, 1)
         } else {
           ptx::tmem_ld_wait();
         }
-        if (c + kChunkStep >= kOutCols / 64) {
+        if (c + kChunkStep >= chunks) {
           // Accumulator fully read by this warp: hand it back to the (leader's) MMA warp.
           ptx::tc_fence_before_sync();
           __syncwarp();
@@ -438,7 +469,7 @@ __global__ void __launch_bounds__(kPlainThreads, 1)
             *reinterpret_cast<uint4*>(cbuf + lr * 128 + (((lane & 7) ^ (lr & 7)) * 16)) = res[i];
           }
           __syncwarp();
-          if (c + kChunkStep < kOutCols / 64) load_residual(c + kChunkStep);
+          if (c + kChunkStep < chunks) load_residual(c + kChunkStep);
         }
         // Row `lane` of the warp's slice, 16-byte pieces swizzled as the tensor store expects.
 #pragma unroll

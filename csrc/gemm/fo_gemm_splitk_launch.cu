@@ -91,10 +91,12 @@ KernelCost kernel_cost(const AlgoConfig& c) {
 
 double plain_time(const GemmParams& p, int algo, bool bf16, int num_kb) {
   const AlgoConfig c = algo_config(algo);
-  const int rows = (c.cta2 ? 2 : 1) * c.mt;  // 128-row tiles of a scheduling unit
-  const int units = (p.tiles_m + rows - 1) / rows * (p.N / c.bn);
+  const int units = plain_units(p, algo);
   const int slots = std::max(1, gemm_max_resident_ctas(algo, bf16, false) / (c.cta2 ? 2 : 1));
   const KernelCost k = kernel_cost(c);
+  if (c.cta2 && c.mt == 1 && c.bn == 256 && plain_tail(units, slots) > 0) {
+    return num_kb * (units / slots * k.per_kb + 0.247);  // the last wave in halves
+  }
   return (units + slots - 1) / slots * (num_kb * k.per_kb + k.epilogue);
 }
 

@@ -336,6 +336,16 @@ void OverlapImpl::run_plain(const at::Tensor& A, const at::Tensor& B, void* out,
   const int pair = c.cta2 ? 2 : 1;
   const int ctas = (p.tiles_m + pair - 1) / pair * pair * p.tiles_n;
   const int grid = std::max(1, std::min(std::min(grid_cap, resident), ctas));
+  const int units = plain_units(p, plan.algo);
+  p.tail_start = units;
+  if (c.cta2 && c.mt == 1 && c.bn == 256 && p.signal == 0 && p.monitor == 0 && opt_exact_algo_ == 0) {
+    const int tail = plain_tail(units, std::max(1, grid / 2));
+    if (tail > 0) {
+      p.tail_start = units - tail;
+      const std::string e = encode_tmap_16bit(&maps.b[1], B.data_ptr(), p.N, p.K, bn / 4);
+      FO_CHECK(e.empty(), "B: ", e);
+    }
+  }
   cuda_check(launch_gemm(plan.algo, bf16, false, maps, p, grid, 1, false, stream()), "GEMM launch");
 }
 
@@ -382,6 +392,7 @@ void OverlapImpl::GemmSwiGLU(at::Tensor A, at::Tensor B, at::Tensor C) {
   p.comm = kCommNone;
   p.ws = 1;
   p.epilogue = kEpiSwiGLU;
+  p.tail_start = (p.tiles_m + 1) / 2 * p.tiles_n;
   p.timeout_ns = static_cast<uint64_t>(opt_timeout_ms_) * 1000000ull;
   p.wait_sleep_ns = static_cast<uint32_t>(opt_wait_sleep_ns_);
   p.out[0] = C.data_ptr();

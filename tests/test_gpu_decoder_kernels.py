@@ -78,10 +78,11 @@ def impl(cuda):
     return i
 
 
-# a split over K, one wave of pairs, an odd number of row tiles, N that only 128-wide tiles divide, 512-row units
+# a split over K, one wave of pairs, an odd number of row tiles, N that only 128-wide tiles divide, 512-row units,
+# a last wave of half-width tiles
 @pytest.mark.parametrize("dt", DTYPES)
 @pytest.mark.parametrize("M,N,K,algo", [(128, 1024, 512, 0), (256, 2048, 1000, 1), (640, 5376, 264, 0), (384, 1152, 128, 2),
-                                        (1024, 8192, 192, 3)])
+                                        (1024, 8192, 192, 3), (1280, 4352, 264, 1)])
 def test_gemm_add(cuda, impl, dt, M, N, K, algo):
     a, b = torch.randn(M, K, device=cuda).to(dt), (0.1 * torch.randn(N, K, device=cuda)).to(dt)
     r = torch.randn(M, N, device=cuda).to(dt)
