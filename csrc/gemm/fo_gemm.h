@@ -45,10 +45,12 @@ inline int plain_units(const GemmParams& p, int algo) {
   const int rows = (c.cta2 ? 2 : 1) * c.mt;  // 128-row tiles of a unit
   return (p.tiles_m + rows - 1) / rows * (p.N / c.bn);
 }
-// Units of the last wave that are computed as halves: all of them if their halves fit one wave.
+// Units of the last wave that are computed as halves: all of them if their halves fit one wave.  A
+// problem of less than a wave is left to the kernels with narrow tiles and a deeper operand ring
+// (256 x 8192 x 3584: 23.9 us in halves, 17.1 us).
 inline int plain_tail(int units, int slots) {
   const int tail = units % slots;
-  return 2 * tail <= slots ? tail : 0;
+  return units > slots && 2 * tail <= slots ? tail : 0;
 }
 constexpr int kSplitBN = 128;
 // split: -1 automatic, 0 never, 2 / 4 / 8 that split wherever it fits the device; exact: algo's own kernel.

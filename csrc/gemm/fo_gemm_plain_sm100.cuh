@@ -30,7 +30,7 @@
 // 11.5 -> 10.2 us; 256 x 256 per CTA, whose epilogue is exposed at every tile: 17.4 -> 15.3 us, and
 // 229 -> 200 us at 16384 x 8192 x 1024.
 //
-// Last wave.  With CTA pairs on 256 x 256 tiles the tiles left over after the last full wave are computed
+// Last wave.  With CTA pairs on 256-wide tiles the tiles left over after the last full wave are computed
 // as 256 x 128 halves when those fit one wave (tail_start): the wave then takes 0.64 of a full one.
 // 1920 x 5376 x 1000 (168 units on 74 pairs): 26.2 -> 24.2 us; projection + residual + norm of
 // 2048 x 8192 x 1792 (256 units): 76.7 -> 75.1 us a call.
@@ -115,7 +115,7 @@ __global__ void __launch_bounds__(kPlainThreads, 1)
   const int sched_tiles_m = (p.tiles_m + kRowsPerUnit - 1) / kRowsPerUnit;
   const int sched_tiles = sched_tiles_m * p.tiles_n;
   // Positions from tail_start on are two half-width tiles each, side by side in the schedule.
-  constexpr bool kHalves = CTA2 && MT == 1 && BN == 256 && EPI != kEpiSwiGLU;
+  constexpr bool kHalves = CTA2 && MT == 1 && BN == 256;
   const int sched_len = kHalves ? 2 * sched_tiles - p.tail_start : sched_tiles;
   struct Work {
     TileCoord tc;
@@ -128,7 +128,7 @@ __global__ void __launch_bounds__(kPlainThreads, 1)
     const int pos = w.narrow ? p.tail_start + (i - p.tail_start) / 2 : i;
     w.tc = tile_of_position(pos, sched_tiles_m, p.tiles_n, p.raster_sw);
     w.tc.m = kRowsPerUnit * w.tc.m + MT * static_cast<int>(cta_rank);  // first half; halves follow
-    w.n0 = w.tc.n * kOutCols + (w.narrow ? ((i - p.tail_start) & 1) * (BN / 2) : 0);
+    w.n0 = w.tc.n * kOutCols + (w.narrow ? ((i - p.tail_start) & 1) * (kOutCols / 2) : 0);
     return w;
   };
   int32_t* status = p.status[0];
@@ -210,8 +210,8 @@ __global__ void __launch_bounds__(kPlainThreads, 1)
             // accumulators hold the 128 gate columns and then the 128 up columns.
             const int rank = static_cast<int>(cta_rank);
             if (kHalves && work.narrow) {
-              ptx::tma_load_2d_pair(sb, &maps.b_half, &full_bar[stage], kb * kBK, work.n0 + rank * (L::kBRows / 2),
-                                    p.l2_hint_b);
+              const int b_row = EPI == kEpiSwiGLU ? rank * p.N + work.n0 : work.n0 + rank * (L::kBRows / 2);
+              ptx::tma_load_2d_pair(sb, &maps.b_half, &full_bar[stage], kb * kBK, b_row, p.l2_hint_b);
             } else {
               const int b_row = EPI == kEpiSwiGLU ? rank * p.N + work.n0 : work.n0 + rank * L::kBRows;
               ptx::tma_load_2d_pair(sb, &maps.b, &full_bar[stage], kb * kBK, b_row, p.l2_hint_b);
@@ -346,7 +346,8 @@ __global__ void __launch_bounds__(kPlainThreads, 1)
       const bool exists = tc.m < p.tiles_m;
       // tile of the layout that holds this one: the same, or (out_bn > BN) a wider one
       const int n0 = work.n0;
-      const int chunks = (kHalves && work.narrow ? BN / 2 : kOutCols) / 64;
+      const int out_cols = kHalves && work.narrow ? kOutCols / 2 : kOutCols;
+      const int chunks = out_cols / 64;
       const int t = tc.m * (p.N / p.out_bn) + n0 / p.out_bn;
       const int r = exists ? tile_position(p, t, status) : 0;
 
@@ -423,6 +424,10 @@ __global__ void __launch_bounds__(kPlainThreads, 1)
       constexpr int kChunkStep = MT == 2 ? 1 : 2;
       static_assert(kPlainEpilogueWarps * (kOutCols / 64) * L::kWarpBufBytes <= L::kEpiOffset, "the ring must hold a tile");
       const bool last_tile = pos + num_units >= sched_len;
+      if (EPI == kEpiSwiGLU && ok && wg >= chunks && lane == 0) {
+        // a half-width SwiGLU tile has one chunk: nothing for this warp to read before the hand-back
+        ptx::mbar_arrive_cluster(tmem_empty_addr0 + static_cast<uint32_t>(acc) * 8u);
+      }
 #pragma unroll 1
       for (int c = MT == 2 ? 0 : wg; ok && c < chunks; c += kChunkStep) {
         uint32_t v0[32], v1[32];
@@ -430,8 +435,8 @@ __global__ void __launch_bounds__(kPlainThreads, 1)
         ptx::tmem_ld_32x32b_x32(t_row + c * 64 + 32, v1);
         if constexpr (EPI == kEpiSwiGLU) {
           uint32_t u0[32], u1[32];
-          ptx::tmem_ld_32x32b_x32(t_row + kOutCols + c * 64, u0);
-          ptx::tmem_ld_32x32b_x32(t_row + kOutCols + c * 64 + 32, u1);
+          ptx::tmem_ld_32x32b_x32(t_row + out_cols + c * 64, u0);
+          ptx::tmem_ld_32x32b_x32(t_row + out_cols + c * 64 + 32, u1);
           ptx::tmem_ld_wait();
 #pragma unroll
           for (int i = 0; i < 32; ++i) {

@@ -392,7 +392,6 @@ void OverlapImpl::GemmSwiGLU(at::Tensor A, at::Tensor B, at::Tensor C) {
   p.comm = kCommNone;
   p.ws = 1;
   p.epilogue = kEpiSwiGLU;
-  p.tail_start = (p.tiles_m + 1) / 2 * p.tiles_n;
   p.timeout_ns = static_cast<uint64_t>(opt_timeout_ms_) * 1000000ull;
   p.wait_sleep_ns = static_cast<uint32_t>(opt_wait_sleep_ns_);
   p.out[0] = C.data_ptr();
@@ -406,7 +405,13 @@ void OverlapImpl::GemmSwiGLU(at::Tensor A, at::Tensor B, at::Tensor C) {
   setup_out_map(&maps, 0, C.data_ptr(), &p);
   FO_CHECK(p.tma_out != 0, "C must be 16-byte aligned");
   const int resident = gemm_max_resident_ctas(kPairAlgo, s.bf16, false);
-  const int grid = std::max(2, std::min(resident, (p.tiles_m + 1) / 2 * 2 * p.tiles_n));
+  const int units = (p.tiles_m + 1) / 2 * p.tiles_n;
+  const int grid = std::max(2, std::min(resident, 2 * units));
+  p.tail_start = units - plain_tail(units, grid / 2);
+  if (p.tail_start < units) {
+    e = encode_tmap_16bit(&maps.b[1], B.data_ptr(), s.N, s.K, 64);
+    FO_CHECK(e.empty(), "B: ", e);
+  }
   cuda_check(launch_gemm(kPairAlgo, s.bf16, false, maps, p, grid, 1, false, stream()), "SwiGLU GEMM launch");
 }
 

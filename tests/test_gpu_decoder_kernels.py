@@ -102,7 +102,8 @@ def test_gemm_add(cuda, impl, dt, M, N, K, algo):
 
 
 @pytest.mark.parametrize("dt", DTYPES)
-@pytest.mark.parametrize("M,F_,K", [(128, 128, 64), (256, 1152, 1000), (640, 3584, 264), (4096, 2048, 512)])
+@pytest.mark.parametrize("M,F_,K", [(128, 128, 64), (256, 1152, 1000), (640, 3584, 264), (4096, 2048, 512),
+                                    (1280, 2176, 192), (2560, 4096, 72)])
 def test_gemm_swiglu(cuda, impl, dt, M, F_, K):
     a, w = torch.randn(M, K, device=cuda).to(dt), (0.1 * torch.randn(2 * F_, K, device=cuda)).to(dt)
     out = torch.full((M, F_), float("nan"), device=cuda, dtype=dt)
