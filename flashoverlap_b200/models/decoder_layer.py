@@ -33,7 +33,7 @@ TILE_M = 128
 # epilogue.  Below them the library's small-problem kernels make up for the extra pass, e.g. 9.1 us
 # against 8.3 us for 1024 x 1024 x 2048 + residual and 94 against 89 us for SwiGLU of 1024 tokens, hidden 8192, ffn
 # 3584; above, 24.7 against 26.0 us for 1024 x 4096 x 3584 + residual, 158 against 214 us for 4096 x 8192 x 3584 +
-# residual, 162 against 188 us for SwiGLU of 4096 tokens, hidden 4096.
+# residual, 157 against 188 us for SwiGLU of 4096 tokens, hidden 4096.
 MIN_ADD_ELEMENTS = 4 * 1024 * 1024
 MIN_SWIGLU_TOKENS = 2048
 
