@@ -76,6 +76,8 @@ class TPDecoderLayer(nn.Module):
     ``OverlapImpl`` (required for ``impl="fused"``).
     """
 
+    _one_rank = None      # (device, OverlapImpl) of a one-rank layer that was given none
+
     def __init__(self, cfg: DecoderConfig, rank: int, world: int, batch: int, seq: int, impl: str = "fused",
                  overlap_impl=None, tp_group=None, dtype=torch.bfloat16, device="cuda", algo: int = 0,
                  seed: int = 0, fuse_norm: bool = False):
@@ -167,11 +169,21 @@ class TPDecoderLayer(nn.Module):
         x, weight = tensors[0], tensors[1]
         if x.dtype != weight.dtype or x.shape[0] % 128 or weight.shape[0] % 128 or weight.shape[1] % 8:
             return False
-        if self.ov is None:
-            with torch.cuda.device(x.device):
-                self.ov = torch.classes.flashoverlap_class.OverlapImpl()
-                self.ov.nccl_init(0, 1, [0] * 16)
         return True
+
+    def _rank_gemms(self, device: torch.device):
+        """The object whose GEMMs one rank runs: the caller's, or one made on first use per device."""
+        if self.ov is not None:
+            return self.ov
+        if self._one_rank is None or self._one_rank[0] != device:
+            with torch.cuda.device(device):
+                impl = torch.classes.flashoverlap_class.OverlapImpl()
+                impl.nccl_init(0, 1, [0] * 16)
+            self._one_rank = (device, impl)
+        return self._one_rank[1]
+
+    def __getstate__(self):
+        return {**self.__dict__, "_one_rank": None}      # copies and files of the layer make their own
 
     def _adds(self, x_sp, x, weight) -> bool:
         """Whether the row-parallel projection of ``x`` adds the residual in its epilogue."""
@@ -182,7 +194,7 @@ class TPDecoderLayer(nn.Module):
         """``x_sp`` + the row-parallel projection of ``x``."""
         if self._adds(x_sp, x, weight):
             out = torch.empty_like(x_sp)
-            self.ov.gemm_add(x, weight, x_sp, out, config.fitting_algo(x.shape[0], weight.shape[0], self.algo))
+            self._rank_gemms(x.device).gemm_add(x, weight, x_sp, out, config.fitting_algo(x.shape[0], weight.shape[0], self.algo))
             return out
         return x_sp + self._row_parallel(x, weight)
 
@@ -243,7 +255,7 @@ class TPDecoderLayer(nn.Module):
         # MLP block
         if hn.shape[0] >= MIN_SWIGLU_TOKENS and self.ffn_local % 128 == 0 and self._fused_gemm(hn, self.wgu):
             act = torch.empty((B * S, self.ffn_local), dtype=hn.dtype, device=hn.device)
-            self.ov.gemm_swiglu(hn, self.wgu, act)
+            self._rank_gemms(hn.device).gemm_swiglu(hn, self.wgu, act)
             return self._add_row_parallel(h_sp, act, self.wd)
         gu = torch.matmul(hn, self.wgu.t())
         gate, up = gu.split([self.ffn_local, self.ffn_local], dim=-1)

@@ -116,3 +116,20 @@ def test_gemm_swiglu(cuda, impl, dt, M, F_, K):
     mag = a.double().abs() @ w.double().abs().t()
     bound = 0.51 * ULP[dt] * ref.abs() + 2.0 ** -18 * (1.1 * mag[:, :F_] * u.abs() + F.silu(g).abs() * mag[:, F_:]) + 2.0 ** -24
     assert ((out.double() - ref).abs() <= bound).all()
+
+
+def test_one_rank_layer_copies_after_a_call(cuda):
+    """The GEMM object that a one-rank layer makes for itself stays out of its copies."""
+    import copy
+    from flashoverlap_b200.models import DecoderConfig, TPDecoderLayer
+    cfg = DecoderConfig(hidden=2048, ffn=1024, n_heads=4, n_kv_heads=2)
+    layer = TPDecoderLayer(cfg, 0, 1, 1, 2048, impl="fused", device=cuda)
+    x = torch.randn(2048, 2048, device=cuda).to(torch.bfloat16)
+    with torch.no_grad():
+        y = layer(x)
+        assert torch.equal(copy.deepcopy(layer)(x), y)
+    for p in layer.parameters():                       # with a graph to record: the operators that have gradients
+        p.grad = None
+    z = layer(x)
+    z.float().sum().backward()
+    assert layer.wd.grad is not None and (z - y).abs().max() <= 0.02 * y.abs().max()
