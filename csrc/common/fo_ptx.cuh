@@ -30,9 +30,9 @@ FO_DEVICE uint32_t cluster_ctarank() {
 FO_DEVICE void cluster_arrive_release() {
   asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
 }
-// Arrive without memory ordering: enough where the barrier only separates phases of execution, or
-// where a narrower fence (mbar_fence_init) has ordered what the others must see.  The release form
-// waits for every global store this thread has in flight.
+// Arrive without memory ordering: enough only where the barrier separates phases of execution and
+// no word in memory is handed over by it.  The release form waits for every global store this
+// thread has in flight.
 FO_DEVICE void cluster_arrive_relaxed() {
   asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory");
 }

@@ -163,9 +163,10 @@ __global__ void __launch_bounds__(kPlainThreads, 1)
   }
   ptx::tc_fence_before_sync();
   if constexpr (CTA2) {
-    // Both CTAs' barriers must be initialised before either receives a remote signal
-    // (mbar_fence_init has published them).
-    ptx::cluster_arrive_relaxed();
+    // Both CTAs' barriers must be initialised before either receives a remote signal.  The release
+    // form, since this is also what hands s_tmem_base and s_abort to the other warps (no store is in
+    // flight yet that it would wait for).
+    ptx::cluster_arrive_release();
     ptx::cluster_wait_acquire();
   } else {
     __syncthreads();

@@ -1,0 +1,26 @@
+"""Ordering rules of the GEMM kernels that no run can show to be kept, read off their sources."""
+import re
+from pathlib import Path
+
+import pytest
+
+GEMM = Path(__file__).resolve().parent.parent / "csrc" / "gemm"
+KERNELS = ["fo_gemm_plain_sm100.cuh", "fo_gemm_sm100.cuh", "fo_gemm_splitk_sm100.cuh"]
+
+
+def _code(name):
+    return re.sub(r"//[^\n]*", "", (GEMM / name).read_text())
+
+
+@pytest.mark.parametrize("name", KERNELS)
+def test_tmem_base_is_read_behind_an_ordering_barrier(name):
+    """tcgen05.alloc writes the TMEM address to shared memory, and one thread clears the abort flag: the
+    barrier between them and their readers must order memory (a CTA barrier or a cluster barrier's
+    release form), in every branch."""
+    code = _code(name)
+    begin, end = code.index("tmem_alloc"), code.index("tmem_base = *s_tmem_base")
+    setup = code[code.rindex("tmem_relinquish", begin, end):end]
+    pair, _, single = setup.partition("} else {") if "if constexpr (CTA2)" in setup else (setup, "", setup)
+    for branch in (pair, single):
+        barriers = re.findall(r"cluster_arrive_\w+|__syncthreads", branch)
+        assert barriers and barriers[0] in ("__syncthreads", "cluster_arrive_release"), barriers
