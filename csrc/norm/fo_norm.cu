@@ -12,7 +12,6 @@
 
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
-#include <algorithm>
 #include <cstdint>
 
 #include "../common/fo_ptx.cuh"
@@ -85,16 +84,22 @@ __device__ __forceinline__ size_t reordered_offset(int b, int col, int dim, int 
          (col % BN);
 }
 
+// CTAs per SM of the build without prefetch (a full set of warps for rows of up to 4096 elements, but the
+// carve-out that leaves the most L1 holds the reserved shared memory of seven).
+constexpr int norm_ctas_per_sm(int vpt) { return vpt <= 2 ? 7 : (vpt <= 4 ? 6 : 3); }
+
 // Each CTA takes a contiguous block of rows; each thread owns VPT 16-byte vectors of a row
-// (VPT * 256 * 8 >= dim).  Bound by memory.  Row-major input: the next row's vectors are requested
-// before the current row is reduced (register double buffer).  Tile-contiguous input: a CTA's first
-// loads wait for the look-ups of its tiles through RA, which more CTAs per SM hide better than a
-// row of prefetch in each (six of 40 registers a thread instead of four of 64); the look-up is done
-// only when the block of rows crosses into another row panel, not per row.  16384 x 8192 in tiles of
-// 64 x 256: 93.4 -> 88.6 us, 4096 x 4096: 17.9 -> 14.6 us, 8192 x 16384: 106.8 -> 98.7 us.
-template <bool BF16, bool REORDER, int VPT>
-__global__ void __launch_bounds__(kNormThreads, REORDER ? (VPT <= 2 ? 8 : (VPT <= 4 ? 6 : 3))
-                                                        : (VPT <= 2 ? 6 : (VPT <= 4 ? 4 : 2)))
+// (VPT * 256 * 8 >= dim).  Bound by memory.  PREFETCH: the weights stay in registers and the next row's
+// vectors are requested before the current row is reduced (register double buffer).  Without: a
+// tile-contiguous CTA's first loads wait for the look-ups of its tiles through RA, which more CTAs per
+// SM hide better than a row of prefetch in each (six of 40 registers a thread instead of four of 64);
+// the look-up is done only when the block of rows crosses into another row panel, not per row.
+// 16384 x 8192 in tiles of 64 x 256: 93.4 -> 88.6 us, 4096 x 4096: 17.9 -> 14.6 us, 8192 x 16384: 106.8 -> 98.7 us.
+// Few rows fit the machine at once either way, and there the weights' latency behind the reduction
+// is what the second build adds: 64 x 8192 3.6 against 4.3 us, 2048 x 8192 15.7 against 17.4 us.
+template <bool BF16, bool REORDER, int VPT, bool PREFETCH>
+__global__ void __launch_bounds__(kNormThreads, !PREFETCH ? (VPT <= 2 ? 8 : norm_ctas_per_sm(VPT))
+                                                          : (VPT <= 2 ? 6 : (VPT <= 4 ? 4 : 2)))
     rmsnorm_kernel(const uint16_t* __restrict__ X, uint16_t* __restrict__ Y,
                    const uint16_t* __restrict__ W, int rows, int dim, int BM, int BN, int rldn,
                    const int* __restrict__ RA, float eps) {
@@ -107,9 +112,9 @@ __global__ void __launch_bounds__(kNormThreads, REORDER ? (VPT <= 2 ? 8 : (VPT <
   ptx::grid_wait();
   if (row_begin >= row_end) return;
 
-  // Row-major input: the weights stay in registers.  Tile-contiguous: re-read from L1 per row.
+  // Without PREFETCH the weights are re-read from L1 per row.
   [[maybe_unused]] uint4 wv[VPT];
-  if constexpr (!REORDER) {
+  if constexpr (PREFETCH) {
 #pragma unroll
     for (int i = 0; i < VPT; ++i) {
       const int j = threadIdx.x + i * kNormThreads;
@@ -153,12 +158,12 @@ __global__ void __launch_bounds__(kNormThreads, REORDER ? (VPT <= 2 ? 8 : (VPT <
 
   uint4 cur[VPT];
   [[maybe_unused]] uint4 nxt[VPT];
-  if constexpr (!REORDER) load_row(row_begin, cur);
+  if constexpr (PREFETCH) load_row(row_begin, cur);
   for (int b = row_begin; b < row_end; ++b) {
-    if constexpr (REORDER) {
-      load_row(b, cur);
-    } else {
+    if constexpr (PREFETCH) {
       if (b + 1 < row_end) load_row(b + 1, nxt);
+    } else {
+      load_row(b, cur);
     }
     float ss = 0.f;
 #pragma unroll
@@ -180,10 +185,10 @@ __global__ void __launch_bounds__(kNormThreads, REORDER ? (VPT <= 2 ? 8 : (VPT <
       const int j = threadIdx.x + i * kNormThreads;
       if (j < nvec) {
         uint4 w;
-        if constexpr (REORDER) {
-          w = __ldg(reinterpret_cast<const uint4*>(W + static_cast<size_t>(j) * 8));
-        } else {
+        if constexpr (PREFETCH) {
           w = wv[i];
+        } else {
+          w = __ldg(reinterpret_cast<const uint4*>(W + static_cast<size_t>(j) * 8));
         }
         uint4 y;
         y.x = scale_mul2<BF16>(cur[i].x, w.x, scale);
@@ -193,7 +198,7 @@ __global__ void __launch_bounds__(kNormThreads, REORDER ? (VPT <= 2 ? 8 : (VPT <
         __stcs(reinterpret_cast<uint4*>(Y + static_cast<size_t>(b) * dim + static_cast<size_t>(j) * 8), y);
       }
     }
-    if constexpr (!REORDER) {
+    if constexpr (PREFETCH) {
 #pragma unroll
       for (int i = 0; i < VPT; ++i) cur[i] = nxt[i];
     }
@@ -376,6 +381,33 @@ int row_grid(int rows, int sm_count) {
 // The same with `per` rows per CTA (down to one while that leaves the machine short of CTAs).
 int row_grid(int rows, int sm_count, int per) { return rows <= sm_count * 8 ? rows : (rows + per - 1) / per; }
 
+// Blocks of rows for the norm without prefetch, whose CTAs take about as long as they have rows: the
+// number of rows that leaves the least of the last wave idle (`resident` CTAs run at once).
+// 11248 x 1024: 5 -> 21.9, 6 -> 19.7, 8 -> 22.6, 10 -> 26.2 us; 6784 x 640: 6 -> 15.8, 7 -> 11.6; 2608 x 16384: 1 -> 46, 5 -> 44,
+// 6 -> 35, 8 -> 37.  Up to 8 rows (ten where a CTA has an SM's third); five at most for rows of
+// 4097..8192 elements, four if that is as good (16384 x 8192: 4 -> 87, 5 -> 89, 8 -> 92).  One wave of
+// up to 16 narrow rows if it is nearly full (16384 x 256: 8 -> 21.5, 16 -> 20.5; not so 13568 x 768: 7 -> 21.8, 14 -> 22.4).
+int whole_wave_grid(int rows, int resident, int vpt, int dim) {
+  const int single = (rows + resident - 1) / resident;
+  if (dim <= 1024 && single > 8 && single <= 16 && rows >= 0.97 * single * resident) return (rows + single - 1) / single;
+  const bool wide = vpt > 2 && vpt <= 4;
+  // candidates, the preferred of equals first
+  static constexpr int kWide[] = {4, 5, 3};
+  const int first = vpt <= 2 ? 8 : 10, count = wide ? 3 : first;
+  int best = 1;
+  int64_t least = INT64_MAX;
+  for (int i = 0; i < count; ++i) {
+    const int per = wide ? kWide[i] : first - i;
+    const int64_t ctas = (rows + per - 1) / per;
+    const int64_t cost = (ctas + resident - 1) / resident * (wide ? per : per + 1);  // + 1: a wave's start
+    if (cost < least) {
+      least = cost;
+      best = per;
+    }
+  }
+  return (rows + best - 1) / best;
+}
+
 template <bool BF16>
 cudaError_t launch_add_norm(const void* X, const void* T, void* H, void* Y, const void* W, int rows, int dim,
                             float eps, int sm_count, cudaStream_t stream) {
@@ -405,20 +437,36 @@ cudaError_t launch_norm(const void* X, void* Y, const void* W, int rows, int dim
   const int vpt = (nvec + kNormThreads - 1) / kNormThreads;
   // Measured (us, rows per CTA -> time).  Row-major, 8192 x 8192: 2 -> 42.9, 4 -> 45.9, 8 -> 47.6, and the
   // same order at 4096 x 4096 and 8192 x 16384; rows of up to 2048 elements want more (16384 x 2048:
-  // 2 -> 29.3, 7 -> 27.6).  Tile-contiguous: 8192 x 8192 2 -> 49.0, 4 -> 49.4, 8 -> 55.8; 4096 x 8192 2 -> 28.0,
-  // 4 -> 30.6; 16384 x 2048 4 -> 35.4, 8 -> 34.0; 16384 x 512 4 -> 25.3, 16 -> 23.1.
+  // 2 -> 29.3, 7 -> 27.6).
+  // Tile-contiguous: the build with prefetch up to where the other one has gained on it in every place
+  // measured (cold, behind the input's producer, before the output's consumer): 20 rows per SM, 17
+  // for rows over 4096 elements (2048 x 8192: 15.7 against 17.4 us; 2608 x 8192: 21.1 against 19.1 us),
+  // 2 over 8192 (400 x 16384: 12.7 against 9.8 us).  Of fewer, narrow rows that nearly fill their last
+  // wave are the other one's too (1008 x 1024: 3.5 against 3.0 us; 1408 x 1024, 0.68 of two waves: 3.8 against 4.1 us).
+  const int wave = sm_count * norm_ctas_per_sm(vpt);
+  bool prefetch = !REORDER || rows < sm_count * (vpt <= 2 ? 20 : (vpt <= 4 ? 17 : 2));
+  if (REORDER && vpt <= 2 && rows >= 0.86 * wave * ((rows + wave - 1) / wave)) prefetch = false;
   int grid = row_grid(rows, sm_count);
-  if (REORDER) {
-    const int per = vpt > 2 ? std::min(4, rows / 2048) : std::min(vpt == 2 ? 8 : 16, rows / 1024);
-    grid = row_grid(rows, sm_count, std::max(1, per));
+  if (!prefetch) {
+    grid = whole_wave_grid(rows, wave, vpt, dim);
+  } else if (REORDER) {
+    // two rows each as soon as one each takes more than a wave (1008 x 4608: 8.2 -> 6.9 us)
+    const int resident = sm_count * (vpt <= 2 ? 6 : (vpt <= 4 ? 4 : 2));
+    if (grid == rows && rows > resident) grid = (rows + 1) / 2;
   } else if (vpt > 1) {
     grid = row_grid(rows, sm_count, 2);
   }
   const uint16_t* x = static_cast<const uint16_t*>(X);
   uint16_t* y = static_cast<uint16_t*>(Y);
   const uint16_t* w = static_cast<const uint16_t*>(W);
-#define FO_LAUNCH_NORM(V)                                                                      \
-  return launch_rows<rmsnorm_kernel<BF16, REORDER, V>>(grid, stream, x, y, w, rows, dim, BM, BN, rldn, RA, eps)
+#define FO_LAUNCH_NORM(V)                                                                                          \
+  do {                                                                                                             \
+    if constexpr (REORDER) {                                                                                       \
+      if (!prefetch)                                                                                               \
+        return launch_rows<rmsnorm_kernel<BF16, true, V, false>>(grid, stream, x, y, w, rows, dim, BM, BN, rldn, RA, eps); \
+    }                                                                                                              \
+    return launch_rows<rmsnorm_kernel<BF16, REORDER, V, true>>(grid, stream, x, y, w, rows, dim, BM, BN, rldn, RA, eps); \
+  } while (0)
   if (vpt <= 1) {
     FO_LAUNCH_NORM(1);
   } else if (vpt <= 2) {

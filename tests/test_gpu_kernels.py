@@ -550,3 +550,20 @@ def test_reducescatter_rmsnorm_tail_pull_loopback(cuda, ws, algo):
     for r in range(ws):
         y_ref = ops.rmsnorm(plain[r], w, 1e-5).float()
         assert (Y[r].float() - y_ref).abs().max().item() <= 0.02 * y_ref.abs().max().item() + 1e-3, r
+
+
+# both builds of the kernel and every way its rows are dealt out, on either side of where they change: rows that one
+# and two waves hold, the last wave nearly full and not, one wave of many narrow rows; 1, 2, 4 and 8 vectors a thread
+@pytest.mark.parametrize("dim,BN,rows", [(256, 256, (16, 880, 896, 1040, 1792, 2064, 2080, 2944, 2960, 5696, 9568, 16384)),
+                                         (2048, 128, (1024, 2960, 11248)), (2304, 256, (1024, 1776, 2944, 4288)),
+                                         (4608, 128, (592, 608, 1184, 1200, 2512, 2528, 4096, 6000)),
+                                         (16384, 256, (288, 304, 608, 2224, 4096))])
+def test_unreorder_rmsnorm_over_row_counts(cuda, dim, BN, rows):
+    dt = torch.bfloat16
+    w = (1 + 0.1 * torch.randn(dim, device=cuda)).to(dt)
+    for n in rows:
+        x = torch.randn(n, dim, device=cuda).to(dt)
+        RA = torch.randperm((n // 16) * (dim // BN), device=cuda, dtype=torch.int32)
+        y = torch.full_like(x, float("nan"))
+        torch.ops.flashoverlap_op.reorder_rmsnorm_eps(ops.reorder(x, 16, BN, RA, 1), y, w, 16, BN, 1, RA, 1e-5)
+        assert torch.equal(y, ops.rmsnorm(x, w, 1e-5)), n        # the same sums in the same order
