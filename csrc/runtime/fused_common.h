@@ -55,6 +55,13 @@ inline void check_out(const at::Tensor& C, const at::Tensor& A, int64_t numel, c
   FO_CHECK(C.numel() >= numel, name, " is too small: needs ", numel, " elements");
 }
 
+// Whether the first `a_numel` elements of `a` share memory with the first `b_numel` of `b`.
+inline bool overlaps(const at::Tensor& a, int64_t a_numel, const at::Tensor& b, int64_t b_numel) {
+  const auto a0 = reinterpret_cast<uintptr_t>(a.data_ptr()), b0 = reinterpret_cast<uintptr_t>(b.data_ptr());
+  return a0 < b0 + static_cast<uintptr_t>(b_numel) * b.element_size() &&
+         b0 < a0 + static_cast<uintptr_t>(a_numel) * a.element_size();
+}
+
 inline const int* int_ptr_or_null(const at::Tensor& t, const char* name) {
   if (!t.defined() || t.numel() == 0) return nullptr;
   FO_CHECK(t.is_cuda() && t.scalar_type() == at::kInt && t.is_contiguous(), name,

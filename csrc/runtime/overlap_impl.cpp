@@ -363,6 +363,9 @@ void OverlapImpl::GemmAdd(at::Tensor A, at::Tensor B, at::Tensor R, at::Tensor C
   check_out(C, A, static_cast<int64_t>(s.M) * s.N, "C");
   check_out(R, A, static_cast<int64_t>(s.M) * s.N, "R");
   FO_CHECK(reinterpret_cast<uintptr_t>(R.data_ptr()) % 16 == 0, "R must be 16-byte aligned");
+  const int64_t numel = static_cast<int64_t>(s.M) * s.N;
+  FO_CHECK(!overlaps(C, numel, A, A.numel()) && !overlaps(C, numel, B, B.numel()), "C must not overlap A or B");
+  FO_CHECK(C.data_ptr() == R.data_ptr() || !overlaps(C, numel, R, numel), "C must be R or not overlap it");
   run_plain(A, B, C.data_ptr(), kOutNatural, nullptr, nullptr, 1, nullptr, 0, false, false, nullptr,
             0, static_cast<int>(Algo), sm_count_, R.data_ptr());
 }
@@ -376,6 +379,8 @@ void OverlapImpl::GemmSwiGLU(at::Tensor A, at::Tensor B, at::Tensor C) {
   FO_CHECK(s.M % kBM == 0 && s.N % 256 == 0 && s.K % 8 == 0, "gemm_swiglu needs M a multiple of 128, ",
            "B of 2 * N rows with N a multiple of 128, and K a multiple of 8 (M=", s.M, " rows of B=", s.N, " K=", s.K, ")");
   check_out(C, A, static_cast<int64_t>(s.M) * f, "C");
+  const int64_t numel = static_cast<int64_t>(s.M) * f;
+  FO_CHECK(!overlaps(C, numel, A, A.numel()) && !overlaps(C, numel, B, B.numel()), "C must not overlap A or B");
   constexpr int kPairAlgo = 1;  // CTA pairs, 256-wide B tiles, strips of 8
   GemmTensorMaps maps;
   GemmParams p;
@@ -713,7 +718,14 @@ void OverlapImpl::GemmReduceScatterAddRmsNormFused(at::Tensor A, at::Tensor B, a
     check_out(R, A, static_cast<int64_t>(s.M) * s.N, "R");
     check_out(Y, A, static_cast<int64_t>(s.M) * s.N, "Y");
     at::Tensor r2 = R.view({s.M, s.N});
-    GemmAdd(A, B, r2, r2, Algo);
+    if (overlaps(R, R.numel(), A, A.numel()) || overlaps(R, R.numel(), B, B.numel())) {
+      // x += x W^T: finished tiles must not replace operands that later tiles still load
+      at::Tensor sum = at::empty_like(r2);
+      GemmAdd(A, B, r2, sum, Algo);
+      r2.copy_(sum);
+    } else {
+      GemmAdd(A, B, r2, r2, Algo);
+    }
     cuda_check(rmsnorm_launch(r2.data_ptr(), Y.data_ptr(), W.data_ptr(), s.M, s.N, static_cast<float>(eps), s.bf16,
                               sm_count_, stream()),
                "rmsnorm");

@@ -67,7 +67,7 @@ class OverlapImpl : public torch::CustomClassHolder {
   void GemmReduceScatterAddRmsNormFused(at::Tensor A, at::Tensor B, at::Tensor R, at::Tensor Y, at::Tensor W,
                                         double eps, int64_t Algo);
   // Single-rank GEMMs with what follows them in a transformer block done in the epilogue:
-  //   C <- A * B^T + R        (R row-major like C; C may be R)
+  //   C <- A * B^T + R        (R row-major like C; C may be R, and overlaps A, B and R in no other way)
   //   C <- silu(A * G^T) * (A * U^T)   B = [G; U], G and U [N, K] each, C [M, N]
   void GemmAdd(at::Tensor A, at::Tensor B, at::Tensor R, at::Tensor C, int64_t Algo);
   void GemmSwiGLU(at::Tensor A, at::Tensor B, at::Tensor C);

@@ -133,3 +133,37 @@ def test_one_rank_layer_copies_after_a_call(cuda):
     z = layer(x)
     z.float().sum().backward()
     assert layer.wd.grad is not None and (z - y).abs().max() <= 0.02 * y.abs().max()
+
+
+# the residual is the projection's input (h += h W^T), a part of it, and the weights' memory
+@pytest.mark.parametrize("dt", DTYPES)
+@pytest.mark.parametrize("where", ["A", "A shifted", "B"])
+def test_add_norm_with_residual_over_an_operand(cuda, impl, dt, where):
+    M, N = 2048, 2048
+    mem = torch.randn(M + 128, N, device=cuda).to(dt)
+    other = (0.1 * torch.randn(M, N, device=cuda)).to(dt)
+    r = mem[64:64 + M] if where == "A shifted" else mem[:M]
+    a, b = (other, mem[:M]) if where == "B" else (mem[:M], other)
+    w, y = torch.ones(N, device=cuda, dtype=dt), torch.empty(M, N, device=cuda, dtype=dt)
+    product = torch.empty_like(y)
+    impl.cutlass_gemm(a, b, product, 1)
+    h = r + product
+    impl.gemm_reducescatter_add_rmsnorm_fused(a, b, r, y, w, 1e-5, 1)
+    impl.check_status()
+    assert torch.equal(r, h) and torch.equal(y, ops.rmsnorm(h, w, 1e-5))
+
+
+def test_epilogue_gemms_refuse_overlapping_outputs(cuda, impl):
+    mem = torch.zeros(1024 * 256, device=cuda, dtype=torch.bfloat16)
+    at = lambda row: mem[row * 256:(row + 256) * 256].view(256, 256)
+    a, b, r, c = at(0), at(256), at(512), at(768)
+    impl.gemm_add(a, b, r, c, 0)
+    for bad in (at(0), at(128), at(384), at(448), at(640)):
+        with pytest.raises(RuntimeError):
+            impl.gemm_add(a, b, r, bad, 0)
+    half = lambda row: mem[row * 256:(row + 128) * 256].view(256, 128)
+    impl.gemm_swiglu(a, b, half(512))
+    for bad in (half(0), half(128), half(256), half(448)):
+        with pytest.raises(RuntimeError):
+            impl.gemm_swiglu(a, b, bad)
+    impl.check_status()
