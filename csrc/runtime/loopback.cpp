@@ -20,7 +20,7 @@ std::vector<int64_t> fused_loopback(std::string comm_op, std::vector<at::Tensor>
                                     c10::optional<at::Tensor> norm_w, double norm_eps,
                                     c10::optional<at::Tensor> trace, int64_t epi_bufs, int64_t pull_direct,
                                     c10::optional<std::vector<at::Tensor>> norm_res,
-                                    c10::optional<std::vector<at::Tensor>> norm_out) {
+                                    c10::optional<std::vector<at::Tensor>> norm_out, int64_t push_lag) {
   const at::Tensor RA = RA_opt.has_value() ? *RA_opt : at::Tensor();
   const at::Tensor cseg_gpu = cseg_opt.has_value() ? *cseg_opt : at::Tensor();
   const int ws = static_cast<int>(A.size());
@@ -104,10 +104,11 @@ std::vector<int64_t> fused_loopback(std::string comm_op, std::vector<at::Tensor>
   p.ws = ws;
   p.rank_base = 0;
   p.strided_rows = strided_rows ? 1 : 0;
-  // Every rank's staging is on this GPU: nothing to hide behind later tiles, and a tile signalled late is
-  // reduced late (2048 x 4096 x 1024 reduce-scattered over four ranks: 102 -> 91 us a launch, eight ranks of 4096 x 8192 x 1024
-  // pushing 596 -> 546 us).
-  p.push_lag = 0;
+  // By default no lag: every rank's staging is on this GPU, so there is nothing to hide behind later
+  // tiles, and a tile signalled late is reduced late (2048 x 4096 x 1024 reduce-scattered over four ranks:
+  // 102 -> 91 us a launch, eight ranks of 4096 x 8192 x 1024 pushing 596 -> 546 us).
+  FO_CHECK(push_lag >= -1 && push_lag <= 4, "push_lag must be -1 (as on several GPUs) or 0..4");
+  p.push_lag = push_lag < 0 ? default_push_lag(p.K) : static_cast<int>(push_lag);
   p.stage_local = stage_local ? 1 : 0;
   p.pull_direct = (stage_local && pull_direct != 0) ? 1 : 0;
   FO_CHECK(epi_bufs == 2 || epi_bufs == 4, "epi_bufs must be 2 or 4");

@@ -26,7 +26,9 @@ namespace fo {
 // load per rank); pull_direct != 0 with it: the epilogue threads store the partial tiles themselves
 // instead of handing them to the push warp's TMA stores.  norm_res / norm_out (with norm_w): per-rank
 // residual added to the reduced rows before they are stored in out[r] and normalised, and per-rank
-// destination of the normalised rows (default: over out[r]).  Returns ws * kStatusWords status words.
+// destination of the normalised rows (default: over out[r]).  push_lag: tiles whose pushes may be in flight
+// before the oldest one's arrival is signalled - 0 (none), 1..4, or -1 for what ranks on several GPUs
+// use at this K.  Returns ws * kStatusWords status words.
 std::vector<int64_t> fused_loopback(std::string comm_op, std::vector<at::Tensor> A,
                                     std::vector<at::Tensor> B, std::vector<at::Tensor> out,
                                     c10::optional<at::Tensor> RA,
@@ -37,6 +39,6 @@ std::vector<int64_t> fused_loopback(std::string comm_op, std::vector<at::Tensor>
                                     c10::optional<at::Tensor> norm_w, double norm_eps,
                                     c10::optional<at::Tensor> trace, int64_t epi_bufs, int64_t pull_direct,
                                     c10::optional<std::vector<at::Tensor>> norm_res,
-                                    c10::optional<std::vector<at::Tensor>> norm_out);
+                                    c10::optional<std::vector<at::Tensor>> norm_out, int64_t push_lag);
 
 }  // namespace fo

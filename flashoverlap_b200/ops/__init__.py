@@ -77,7 +77,7 @@ def fused_loopback(comm_op: str, A: List[torch.Tensor], B: List[torch.Tensor], o
                    norm_eps: float = 1e-5, trace: Optional[torch.Tensor] = None,
                    epi_bufs: int = 2, pull_direct: bool = False,
                    norm_res: Optional[List[torch.Tensor]] = None,
-                   norm_out: Optional[List[torch.Tensor]] = None) -> List[List[int]]:
+                   norm_out: Optional[List[torch.Tensor]] = None, push_lag: int = 0) -> List[List[int]]:
     """All ranks of a fused GEMM+collective on ONE GPU in one cooperative launch (test aid).
 
     ``stage_local`` selects the pull protocol: every rank stages its partial tiles in its own
@@ -91,7 +91,10 @@ def fused_loopback(comm_op: str, A: List[torch.Tensor], B: List[torch.Tensor], o
     ``pull_direct`` (with ``stage_local``): the epilogue threads store the partial tiles into the local
     staging themselves instead of handing every chunk to the push warp's TMA stores.  ``norm_res`` /
     ``norm_out`` (with ``norm_w``): per-rank residual added to the reduced rows before they are stored in
-    ``out[r]`` and normalised, and per-rank destination of the normalised rows (default: over ``out[r]``)."""
+    ``out[r]`` and normalised, and per-rank destination of the normalised rows (default: over ``out[r]``).
+    ``push_lag`` (push protocol): tiles whose stores may be in flight before the oldest one's arrival is
+    signalled - 0 (none: the stores stay on this GPU), 1..4, or -1 for the lag that ranks on several GPUs
+    use at this K."""
     flat = list(_op().fused_loopback(comm_op, A, B, out, RA, cseg, algo, strided_rows, natural_out, repeat,
-                                     timeout_ms, stage_local, mlen, norm_w, norm_eps, trace, epi_bufs, int(pull_direct), norm_res, norm_out))
+                                     timeout_ms, stage_local, mlen, norm_w, norm_eps, trace, epi_bufs, int(pull_direct), norm_res, norm_out, push_lag))
     return [flat[i:i + 8] for i in range(0, len(flat), 8)]

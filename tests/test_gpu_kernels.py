@@ -196,7 +196,7 @@ def test_wait_flag_completes_and_times_out(cuda):
 
 
 def _loopback_case(cuda, comm_op, ws, M, N, K, algo, strided, natural, repeat=1, groups=None, dt=torch.bfloat16,
-                   stage_local=False, epi_bufs=2):
+                   stage_local=False, epi_bufs=2, push_lag=0):
     p = config.algo_params(algo)
     BM, BN = p["BM"], p["BN"]
     tiles = (M // BM) * (N // BN)
@@ -209,7 +209,7 @@ def _loopback_case(cuda, comm_op, ws, M, N, K, algo, strided, natural, repeat=1,
     out = [torch.full((rows, N), float("nan"), device=cuda, dtype=dt) for _ in range(ws)]
     st = ops.fused_loopback(comm_op, A, B, out, RA=RA, cseg=cseg, algo=algo, strided_rows=strided,
                             natural_out=natural, repeat=repeat, timeout_ms=2000, stage_local=stage_local,
-                            epi_bufs=epi_bufs)
+                            epi_bufs=epi_bufs, push_lag=push_lag)
     assert all(s[0] == 0 for s in st), st
     for r in range(ws):
         if comm_op == "all_reduce":
@@ -309,6 +309,28 @@ def test_fused_loopback_four_chunk_buffers(cuda, comm_op):
     _loopback_case(cuda, comm_op, 4, 1024, 2048, 256, 2, False, False, repeat=3, epi_bufs=4)
     _loopback_case(cuda, comm_op, 8, 2048, 2048, 256, 0, True, False, repeat=2, epi_bufs=4)
     _loopback_case(cuda, comm_op, 2, 2048, 2048, 128, 2, True, True, repeat=2, stage_local=True, epi_bufs=4)
+
+
+@pytest.mark.parametrize("lag", [1, 2, 3, 4])
+@pytest.mark.parametrize("comm_op,ws,M,N,algo,kw", [
+    ("all_reduce", 8, 2048, 2048, 0, dict(repeat=3)),
+    ("reduce_scatter", 8, 2048, 2048, 0, dict(epi_bufs=4, repeat=2)),
+    ("all_reduce", 4, 2048, 3072, 2, dict(groups=[100, 200, 84], repeat=2, dt=torch.float16)),
+    ("reduce_scatter", 2, 4096, 6144, 0, dict(epi_bufs=4)),
+])
+def test_fused_loopback_push_lag(cuda, lag, comm_op, ws, M, N, algo, kw):
+    """The push protocol as ranks on several GPUs run it: a tile's arrival is signalled `lag` tiles later."""
+    p = config.algo_params(algo)
+    ctas = torch.cuda.get_device_properties(cuda).multi_processor_count // ws
+    assert (M // p["BM"]) * (N // p["BN"]) > (lag + 1) * ctas        # every CTA's ring fills up and turns over
+    _loopback_case(cuda, comm_op, ws, M, N, 128, algo, ws != 4, ws == 2, push_lag=lag, **kw)
+
+
+def test_fused_loopback_push_lag_by_k_and_refused(cuda):
+    _loopback_case(cuda, "reduce_scatter", 8, 2048, 2048, 2048, 0, False, True, push_lag=-1)
+    for bad in (-2, 5):
+        with pytest.raises(RuntimeError):
+            _loopback_case(cuda, "all_reduce", 2, 512, 512, 64, 0, True, True, push_lag=bad)
 
 
 def test_fused_loopback_eight_ranks(cuda):
