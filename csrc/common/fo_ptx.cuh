@@ -54,10 +54,15 @@ FO_DEVICE void st_shared_cluster_v4(uint32_t cluster_addr, uint32_t x, uint32_t 
                : "memory");
 }
 // Arrive on an mbarrier that may live in another CTA of the cluster (address from mapa_shared).
-// Release at CTA scope (the instruction's default): what the barrier hands over is TMEM, ordered by
-// the tcgen05 fence in front of it, and no global data.  At cluster scope the arrive would first
-// wait for every global store this thread has in flight to reach L2 (about 1,500 cycles).
 FO_DEVICE void mbar_arrive_cluster(uint32_t cluster_addr) {
+  asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(cluster_addr)
+               : "memory");
+}
+// The same where TMEM alone is handed over, which the tcgen05 fence in front of it orders, and no word in
+// memory: release at CTA scope (the instruction's default).  At cluster scope the arrive first waits
+// for every global store this thread has in flight to reach L2 (about 1,500 cycles), which
+// counts where the arriving threads store the tiles themselves.
+FO_DEVICE void mbar_arrive_cluster_tmem(uint32_t cluster_addr) {
   asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(cluster_addr) : "memory");
 }
 

@@ -427,7 +427,7 @@ __global__ void __launch_bounds__(kPlainThreads, 1)
       const bool last_tile = pos + num_units >= sched_len;
       if (EPI == kEpiSwiGLU && ok && wg >= chunks && lane == 0) {
         // a half-width SwiGLU tile has one chunk: nothing for this warp to read before the hand-back
-        ptx::mbar_arrive_cluster(tmem_empty_addr0 + static_cast<uint32_t>(acc) * 8u);
+        ptx::mbar_arrive_cluster_tmem(tmem_empty_addr0 + static_cast<uint32_t>(acc) * 8u);
       }
 #pragma unroll 1
       for (int c = MT == 2 ? 0 : wg; ok && c < chunks; c += kChunkStep) {
@@ -451,7 +451,7 @@ __global__ void __launch_bounds__(kPlainThreads, 1)
           // Accumulator fully read by this warp: hand it back to the (leader's) MMA warp.
           ptx::tc_fence_before_sync();
           __syncwarp();
-          if (lane == 0) ptx::mbar_arrive_cluster(tmem_empty_addr0 + static_cast<uint32_t>(acc) * 8u);
+          if (lane == 0) ptx::mbar_arrive_cluster_tmem(tmem_empty_addr0 + static_cast<uint32_t>(acc) * 8u);
         }
         if (!exists) continue;
         // The buffer is free once the previous store has read it: about 600 cycles after its issue,

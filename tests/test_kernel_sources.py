@@ -24,3 +24,12 @@ def test_tmem_base_is_read_behind_an_ordering_barrier(name):
     for branch in (pair, single):
         barriers = re.findall(r"cluster_arrive_\w+|__syncthreads", branch)
         assert barriers and barriers[0] in ("__syncthreads", "cluster_arrive_release"), barriers
+
+
+def test_fused_kernel_hands_accumulators_back_at_cluster_scope():
+    """The kernels that run over several GPUs keep the arrive that releases at cluster scope; the CTA-scope
+    form is the plain kernel's."""
+    ptx = re.sub(r"//[^\n]*", "", (GEMM.parent / "common" / "fo_ptx.cuh").read_text())
+    body = ptx[ptx.index("void mbar_arrive_cluster("):]
+    assert "mbarrier.arrive.release.cluster.shared::cluster" in body[:body.index("}")]
+    assert "mbar_arrive_cluster(" in _code("fo_gemm_sm100.cuh") and "_tmem(" not in _code("fo_gemm_sm100.cuh")
