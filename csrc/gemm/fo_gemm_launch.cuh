@@ -35,14 +35,14 @@ cudaError_t launch_kernel(Kernel kernel, int threads, int smem, bool* attr_set, 
     ++cfg.numAttrs;
   }
   if (query != nullptr) {
-    cudaDeviceProp prop;
-    cudaError_t e = cudaGetDeviceProperties(&prop, dev);
+    int sm_count = 0;  // one attribute: all of cudaGetDeviceProperties takes milliseconds
+    cudaError_t e = cudaDeviceGetAttribute(&sm_count, cudaDevAttrMultiProcessorCount, dev);
     if (e != cudaSuccess) return e;
     if (!CTA2) {
-      *query = prop.multiProcessorCount;  // shared memory admits exactly one CTA per SM
+      *query = sm_count;  // shared memory admits exactly one CTA per SM
       return cudaSuccess;
     }
-    cfg.gridDim = dim3(prop.multiProcessorCount & ~1, 1, 1);
+    cfg.gridDim = dim3(sm_count & ~1, 1, 1);
     int clusters = 0;
     e = cudaOccupancyMaxActiveClusters(&clusters, kernel, &cfg);
     if (e != cudaSuccess) return e;

@@ -51,9 +51,7 @@ void OverlapImpl::NcclInit(int64_t rank, int64_t world, std::vector<int64_t> id)
   rank_ = static_cast<int>(rank);
   world_ = static_cast<int>(world);
   cuda_check(cudaGetDevice(&device_), "cudaGetDevice");
-  cudaDeviceProp prop;
-  cuda_check(cudaGetDeviceProperties(&prop, device_), "cudaGetDeviceProperties");
-  sm_count_ = prop.multiProcessorCount;
+  sm_count_ = at::cuda::getDeviceProperties(device_)->multiProcessorCount;  // asked once per process: it takes milliseconds
   if (world_ > 1) {
     ncclUniqueId uid = unpack_nccl_id(id);
     FO_NCCL_CHECK(ncclCommInitRank(&comm_, world_, uid, rank_));

@@ -76,7 +76,7 @@ class TPDecoderLayer(nn.Module):
     ``OverlapImpl`` (required for ``impl="fused"``).
     """
 
-    _one_rank = None      # (device, OverlapImpl) of a one-rank layer that was given none
+    _one_rank = None      # (device, OverlapImpl) of a one-rank layer that was given none, see check_status
 
     def __init__(self, cfg: DecoderConfig, rank: int, world: int, batch: int, seq: int, impl: str = "fused",
                  overlap_impl=None, tp_group=None, dtype=torch.bfloat16, device="cuda", algo: int = 0,
@@ -109,6 +109,9 @@ class TPDecoderLayer(nn.Module):
         gn = torch.Generator(device="cpu").manual_seed(seed)        # norm weights are replicated
         self.attn_norm = nn.Parameter((1 + 0.02 * torch.randn(h, generator=gn)).to(dtype).to(device))
         self.mlp_norm = nn.Parameter((1 + 0.02 * torch.randn(h, generator=gn)).to(dtype).to(device))
+
+        if self.world == 1 and impl == "fused" and torch.device(device).type == "cuda":
+            self._rank_gemms(self.wd.device)
 
     # ---- token <-> shard helpers -------------------------------------------------------------
     def shard_rows(self) -> torch.Tensor:
@@ -169,18 +172,30 @@ class TPDecoderLayer(nn.Module):
         x, weight = tensors[0], tensors[1]
         if x.dtype != weight.dtype or x.shape[0] % 128 or weight.shape[0] % 128 or weight.shape[1] % 8:
             return False
-        return True
+        return self._rank_gemms(x.device) is not None
 
     def _rank_gemms(self, device: torch.device):
-        """The object whose GEMMs one rank runs: the caller's, or one made on first use per device."""
+        """The object whose GEMMs one rank runs: the caller's, or one of the layer's own, made with the layer (and
+        again on first use on another device).  None where it would have to be made while a stream
+        is being captured: its status words would belong to the graph."""
         if self.ov is not None:
             return self.ov
         if self._one_rank is None or self._one_rank[0] != device:
+            if torch.cuda.is_current_stream_capturing():
+                return None
+            from .._build import load
+            load()
             with torch.cuda.device(device):
                 impl = torch.classes.flashoverlap_class.OverlapImpl()
                 impl.nccl_init(0, 1, [0] * 16)
             self._one_rank = (device, impl)
         return self._one_rank[1]
+
+    def check_status(self) -> None:
+        """Raises if a kernel of this layer's GEMM object gave up a wait (its outputs are then incomplete)."""
+        for impl in (self.ov, self._one_rank[1] if self._one_rank is not None else None):
+            if impl is not None:
+                impl.check_status()
 
     def __getstate__(self):
         return {**self.__dict__, "_one_rank": None}      # copies and files of the layer make their own

@@ -133,6 +133,7 @@ def test_one_rank_layer_copies_after_a_call(cuda):
     z = layer(x)
     z.float().sum().backward()
     assert layer.wd.grad is not None and (z - y).abs().max() <= 0.02 * y.abs().max()
+    layer.check_status()
 
 
 # the residual is the projection's input (h += h W^T), a part of it, and the weights' memory
@@ -167,3 +168,60 @@ def test_epilogue_gemms_refuse_overlapping_outputs(cuda, impl):
         with pytest.raises(RuntimeError):
             impl.gemm_swiglu(a, b, bad)
     impl.check_status()
+
+
+def _one_rank_layer(cuda, T=2048):
+    from flashoverlap_b200.models import DecoderConfig, TPDecoderLayer
+    cfg = DecoderConfig(hidden=2048, ffn=1024, n_heads=4, n_kv_heads=2)
+    return TPDecoderLayer(cfg, 0, 1, 1, T, impl="fused", device=cuda), torch.randn(T, 2048, device=cuda).to(torch.bfloat16)
+
+
+def test_one_rank_layer_makes_its_gemm_object_with_itself(cuda):
+    """No set-up is left for the first forward, and a capture of that first forward holds no set-up either."""
+    layer, x = _one_rank_layer(cuda)
+    device, made = layer._one_rank
+    with torch.no_grad():
+        layer.check_status()
+        g = torch.cuda.CUDAGraph()
+        torch.cuda.synchronize()
+        with torch.cuda.graph(g):
+            y = layer(x)
+        layer.check_status()                       # the words are not the graph's: valid before any replay
+        g.replay()
+        assert torch.equal(y, layer(x))
+    assert layer._one_rank[1] is made and device == x.device
+    layer.check_status()
+
+
+def test_one_rank_layer_copy_first_called_under_capture(cuda):
+    """A copy has no object yet and makes none while a stream is captured: the operators of torch serve."""
+    import copy
+    layer, x = _one_rank_layer(cuda)
+    twin = copy.deepcopy(layer)
+    with torch.no_grad():
+        ref = layer(x)
+        F.scaled_dot_product_attention(*[torch.zeros(1, 4, 64, 128, device=cuda, dtype=x.dtype)] * 3, is_causal=True)
+        torch.matmul(x, twin.wqkv.t())             # the library's own workspaces, ahead of the capture
+        torch.cuda.synchronize()
+        g = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(g):
+            y = twin(x)
+        assert twin._one_rank is None
+        twin.check_status()
+        g.replay()
+    # the two ways round at different places: 2 units of bf16 in the largest element
+    assert (y - ref).abs().max() <= 2.0 ** -6 * ref.abs().max()
+    with torch.no_grad():
+        assert torch.equal(twin(x), ref) and twin._one_rank is not None
+    twin.check_status()
+
+
+def test_layer_check_status_reports_a_wait_that_gave_up(cuda):
+    layer, x = _one_rank_layer(cuda, 128)
+    own = layer._one_rank[1]
+    own.set_option("timeout_ms", 50)
+    own.wait_flag(1, torch.zeros(4, dtype=torch.int32, device=cuda), 2)      # nobody signals
+    with pytest.raises(RuntimeError):
+        layer.check_status()
+    own.reset_status()
+    layer.check_status()

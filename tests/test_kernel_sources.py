@@ -33,3 +33,9 @@ def test_fused_kernel_hands_accumulators_back_at_cluster_scope():
     body = ptx[ptx.index("void mbar_arrive_cluster("):]
     assert "mbarrier.arrive.release.cluster.shared::cluster" in body[:body.index("}")]
     assert "mbar_arrive_cluster(" in _code("fo_gemm_sm100.cuh") and "_tmem(" not in _code("fo_gemm_sm100.cuh")
+
+
+def test_objects_and_launches_query_no_device_properties():
+    """cudaGetDeviceProperties takes milliseconds: not once per object, nor per kernel of a choice."""
+    for path in ("runtime/overlap_impl.cpp", "runtime/loopback.cpp", "gemm/fo_gemm_launch.cuh", "gemm/fo_gemm_splitk_launch.cu"):
+        assert "cudaGetDeviceProperties(" not in re.sub(r"//[^\n]*", "", (GEMM.parent / path).read_text()), path
