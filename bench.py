@@ -363,6 +363,7 @@ def run_ours(args):
         cand, algo_times, cands = (int(tuned["Algo"]), tuned.get("protocol", protocols[-1])), None, None
         if cand[1] not in protocols:
             cand = (cand[0], protocols[-1])
+        impl.set_option("exact_algo", 1 if config.is_measured(tuned) else 0)    # a timed Algo runs as it was timed
     else:
         cands = [(a, pr) for pr in protocols for a in ((19, 3, 17, 1) if world <= 2 else (3, 1, 19, 17))]
         cand, algo_times = pick_algo(torch, dist, world, step_cand, cands, flush, check=healthy)

@@ -13,6 +13,7 @@ import torch.distributed as dist
 import torch.nn as nn
 
 from ..utils import layout
+from ..utils.config import is_measured
 
 
 class RowParallelLayer(nn.Module):
@@ -40,7 +41,9 @@ class RowParallelLayer(nn.Module):
 
 
 class OverlapRowParallelLayer(nn.Module):
-    """``config`` is a tuned JSON dict (BM, BN, Algo, hint, cSeg).
+    """``config`` is a tuned JSON dict (BM, BN, Algo, hint, cSeg), or ``config.default_solution``.  With a
+    timed config (``dur``) an object that this layer makes runs exactly the Algo it names (option
+    ``exact_algo``); otherwise one rank's small or ragged problems may take a faster kernel.
 
     ``layout`` selects what ``forward`` returns:
       * ``"reordered"`` (default, reference behaviour): the tile-contiguous buffer, to be consumed
@@ -72,6 +75,8 @@ class OverlapRowParallelLayer(nn.Module):
             impl.nccl_init(rank, world_size, nccl_id)
             impl.cutlass_init()
             impl.overlap_init()
+            # a timed Algo runs as it was timed; a shared object's setting is its owner's
+            impl.set_option("exact_algo", 1 if is_measured(config) else 0)
         self.overlap_class = impl
         impl.set_option("mode", 0 if mode == "fused" else 1)
 

@@ -122,6 +122,11 @@ def is_tuned(cfg: dict) -> bool:
     return "hint" in cfg and "cSeg" in cfg and not isinstance(cfg.get("Algo"), list)
 
 
+def is_measured(cfg: dict) -> bool:
+    """Whether the config's Algo was timed (a tuner's ``dur``), not picked without a run."""
+    return float(cfg.get("dur", 0.0)) > 0.0
+
+
 def matches(cfg: dict, tp: Optional[int] = None, comm_op: Optional[str] = None, mode: Optional[str] = None) -> bool:
     """Whether a tuned config was searched for this use.  The file name carries only (M, N, K,
     gpu); ``search`` also records the world size, the collective and the overlap mechanism the

@@ -52,6 +52,7 @@ def worker(rank, world, args):
     cfg = config.load_tuned(args.m, args.n, args.k, tp=world, comm_op=args.comm_op, directory=args.path) or \
         config.default_solution(args.m, args.n, args.algo)
     algo = cfg["Algo"]
+    impl.set_option("exact_algo", 1 if config.is_measured(cfg) else 0)      # a timed Algo runs as it was timed
     sm, margin = impl.get_option("sm_count"), impl.get_option("sm_margin")
     res = {"M": args.m, "N": args.n, "K": args.k, "tp": world, "comm_op": args.comm_op, "Algo": algo}
 

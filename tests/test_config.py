@@ -93,3 +93,11 @@ def test_tuned_config_is_used_only_for_what_it_was_tuned_for(tmp_path):
     config.save_solution(path, 128, 256, 0.1, 0, list(range(16)), [16], 1)
     assert config.load_tuned(M, N, K, tp=2, comm_op="reduce_scatter", mode="fused", gpu="b200", directory=tmp_path) is not None
     assert config.load_tuned(M + 128, N, K, gpu="b200", directory=tmp_path) is None
+
+
+def test_is_measured(tmp_path):
+    assert not config.is_measured(config.default_solution(1024, 2048, algo=1))
+    path = tmp_path / "cfg.json"
+    config.save_solution(path, 128, 256, 0.125, 3, [0, 1], [2])
+    assert config.is_measured(config.load_config(path))
+    assert not config.is_measured({"Algo": 3, "BM": 128, "BN": 256, "hint": [0], "cSeg": [1]})

@@ -574,6 +574,26 @@ def test_reducescatter_rmsnorm_tail_pull_loopback(cuda, ws, algo):
         assert (Y[r].float() - y_ref).abs().max().item() <= 0.02 * y_ref.abs().max().item() + 1e-3, r
 
 
+def test_row_parallel_layer_runs_a_timed_algo_as_it_was_timed(cuda):
+    from flashoverlap_b200.models import OverlapRowParallelLayer
+    M, N, K = 128, 1024, 1024                    # a shape that another kernel is expected to be faster at
+    cfg = config.default_solution(M, N, 0)
+    ids = [0] * 16
+    assert OverlapRowParallelLayer(0, 1, K, N, M, cfg, "all_reduce", ids).overlap_class.get_option("exact_algo") == 0
+    timed = dict(cfg, dur=0.01)
+    layer = OverlapRowParallelLayer(0, 1, K, N, M, timed, "all_reduce", ids, layout_mode="natural")
+    assert layer.overlap_class.get_option("exact_algo") == 1
+    shared = ops.OverlapImpl()
+    shared.nccl_init(0, 1, ids)
+    OverlapRowParallelLayer(0, 1, K, N, M, timed, "all_reduce", ids, impl=shared)
+    assert shared.get_option("exact_algo") == 0  # a shared object's setting stays its owner's
+    x = _rand((M, K), torch.bfloat16, cuda)
+    with torch.no_grad():
+        expect = x.float() @ layer.weight.float().t()
+        assert (layer(x).float() - expect).abs().max().item() <= _tol(expect)
+    layer.overlap_class.check_status()
+
+
 # both builds of the kernel and every way its rows are dealt out, on either side of where they change: rows that one
 # and two waves hold, the last wave nearly full and not, one wave of many narrow rows; 1, 2, 4 and 8 vectors a thread
 @pytest.mark.parametrize("dim,BN,rows", [(256, 256, (16, 880, 896, 1040, 1792, 2064, 2080, 2944, 2960, 5696, 9568, 16384)),
