@@ -141,6 +141,9 @@ int64_t OverlapImpl::GetOption(std::string name) {
   if (name == "tma_out") return opt_tma_out_;
   if (name == "exact_algo") return opt_exact_algo_;
   if (name == "split_k") return opt_split_k_;
+  if (name == "last_algo") return last_algo_;
+  if (name == "last_split") return last_split_;
+  if (name == "last_tail") return last_tail_;
   if (name == "validate") return opt_validate_;
   if (name == "wait_sleep_ns") return opt_wait_sleep_ns_;
   if (name == "pull_direct") return opt_pull_direct_;
@@ -310,6 +313,9 @@ void OverlapImpl::run_plain(const at::Tensor& A, const at::Tensor& B, void* out,
   p.res = res;
   const PlainPlan plan =
       choose_plain(p, algo, bf16, static_cast<int>(opt_split_k_), opt_exact_algo_ != 0);
+  last_algo_ = plan.algo;
+  last_split_ = plan.split;
+  last_tail_ = 0;
   const AlgoConfig c = algo_config(plan.algo);
   const int bn = plan.split != 0 ? kSplitBN : c.bn;
   const int b_rows = plan.split == 0 && c.cta2 ? bn / 2 : bn;
@@ -340,6 +346,7 @@ void OverlapImpl::run_plain(const at::Tensor& A, const at::Tensor& B, void* out,
     const int tail = plain_tail(units, std::max(1, grid / 2));
     if (tail > 0) {
       p.tail_start = units - tail;
+      last_tail_ = tail;
       const std::string e = encode_tmap_16bit(&maps.b[1], B.data_ptr(), p.N, p.K, bn / 4);
       FO_CHECK(e.empty(), "B: ", e);
     }
@@ -411,6 +418,9 @@ void OverlapImpl::GemmSwiGLU(at::Tensor A, at::Tensor B, at::Tensor C) {
   const int units = (p.tiles_m + 1) / 2 * p.tiles_n;
   const int grid = std::max(2, std::min(resident, 2 * units));
   p.tail_start = units - plain_tail(units, grid / 2);
+  last_algo_ = kPairAlgo;
+  last_split_ = 0;
+  last_tail_ = units - p.tail_start;
   if (p.tail_start < units) {
     e = encode_tmap_16bit(&maps.b[1], B.data_ptr(), s.N, s.K, 64);
     FO_CHECK(e.empty(), "B: ", e);

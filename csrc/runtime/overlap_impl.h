@@ -14,6 +14,7 @@
 #include <nccl.h>
 #include <torch/custom_class.h>
 
+#include <atomic>
 #include <memory>
 #include <string>
 #include <vector>
@@ -201,6 +202,9 @@ class OverlapImpl : public torch::CustomClassHolder {
 #else
   int64_t opt_validate_ = 0;     // 1: also check the VALUES of RA / RE / cSEG_GPU (a device-to-host copy per call)
 #endif
+  // What the last plain GEMM ran (read-only options last_algo, last_split, last_tail): the Algo whose
+  // kernel, the CTAs of a split over K (0: none), and the scheduling units computed as halves.
+  std::atomic<int> last_algo_{-1}, last_split_{0}, last_tail_{0};
   int64_t opt_exact_algo_ = 0;   // plain GEMM: 1 runs the Algo's own kernel even where another is faster
   int64_t opt_split_k_ = -1;     // plain GEMM of few tiles split over K: -1 automatic, 0 never, else that many CTAs a tile
   int64_t opt_tma_out_ = -1;     // plain kernels' stores: 0 per-thread stores, else TMA tensor stores where the output allows

@@ -41,6 +41,15 @@ def test_split_gemm_natural(cuda, impl, dt, M, N, K, algo):
             c = torch.full((M, N), float("nan"), device=cuda, dtype=dt)
             impl.cutlass_gemm(a, b, c, algo)
             _check(c, a, b, dt)
+            ran = impl.get_option("last_split")
+            if split >= 0:       # a forced split runs wherever K has that many k-blocks and the clusters fit at once
+                ctas = (M // 128) * (N // 128) * split
+                if split == 0 or (K + 63) // 64 < split or ctas > impl.get_option("sm_count"):
+                    assert ran == 0
+                elif ctas <= impl.get_option("sm_count") * 3 // 4:
+                    assert ran == split
+            elif (M, N, K) == (128, 8192, 3584):
+                assert ran == 2          # the decode batch: 64 tiles, bound by one SM's share of the loads
             again = torch.empty_like(c)
             impl.cutlass_gemm(a, b, again, algo)
             assert torch.equal(c, again)             # the partial sums are added in a fixed order
@@ -64,10 +73,17 @@ def test_split_gemm_reordered(cuda, impl, M, N, K, algo, rldn):
             impl.set_option("split_k", split)
             c = torch.full((M, N), float("nan"), device=cuda, dtype=dt)
             impl.gemm_allreduce_overlap(a, b, c, mm, RA, rldn, e, e.to(cuda), algo, False)
+            small = (M // 128) * (N // 128) * split <= impl.get_option("sm_count") * 3 // 4
+            assert split == -1 or (K + 63) // 64 < split or not small or impl.get_option("last_split") == split
             _check(layout.from_reordered(c.cpu(), M, N, p["BM"], p["BN"], RA.cpu(), rldn).to(cuda), a, b, dt)
     finally:
         impl.set_option("split_k", -1)
     impl.check_status()
+
+
+def _ran(impl):
+    """(Algo whose kernel the last GEMM ran, its split, its units computed as halves)"""
+    return tuple(impl.get_option(name) for name in ("last_algo", "last_split", "last_tail"))
 
 
 # odd row tiles on pairs, 512-row units with nothing to fill them, 256-wide tiles computed as 128-wide ones
@@ -90,8 +106,15 @@ def test_stand_in_kernels(cuda, impl, M, N, K, algo):
             c = torch.full((M, N), float("nan"), device=cuda, dtype=dt)
             impl.cutlass_gemm(a, b, c, algo)
             _check(c, a, b, dt)
+            if exact:
+                assert _ran(impl) == (algo, 0, 0)
+            else:
+                assert _ran(impl)[:2] != (algo, 0)
+                if M == 1920:                            # 168 pair units on 74 pairs: the last 20 in halves
+                    assert _ran(impl)[:2] == (1, 0) and _ran(impl)[2] > 0
             c.fill_(float("nan"))
             impl.gemm_allreduce_overlap(a, b, c, mm, RA, rldn, e, e.to(cuda), algo, False)
+            assert not exact or _ran(impl) == (algo, 0, 0)
             _check(layout.from_reordered(c.cpu(), M, N, p["BM"], p["BN"], RA.cpu(), rldn).to(cuda), a, b, dt)
     finally:
         impl.set_option("exact_algo", 0)
