@@ -120,3 +120,61 @@ def test_stand_in_kernels(cuda, impl, M, N, K, algo):
         impl.set_option("exact_algo", 0)
         impl.set_option("tma_out", -1)
     impl.check_status()
+
+
+# the last wave in halves (80 units on 74 pairs), in a layout whose tiles are twice as wide as the halves; odd row
+# tiles on pairs; 128-wide stand-ins for 256-wide tiles; a split: both types, one and two tiles to a row of the layout
+@pytest.mark.parametrize("dt", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("M,N,K,algo,rldn", [(2560, 2048, 264, 1, 2), (1920, 5376, 136, 0, 1), (256, 8192, 320, 1, 2),
+                                             (512, 4096, 520, 3, 2), (128, 2048, 4096, 0, 2)])
+def test_stand_ins_in_the_tile_contiguous_layout(cuda, impl, dt, M, N, K, algo, rldn):
+    a = (torch.randn(M, K, device=cuda) * 0.5).to(dt)
+    b = (torch.randn(N, K, device=cuda) * 0.5).to(dt)
+    p = config.algo_params(algo)
+    tiles = (M // p["BM"]) * (N // p["BN"])
+    RA = torch.randperm(tiles, device=cuda, dtype=torch.int32)
+    e = torch.empty(0, dtype=torch.int32)
+    mm = torch.zeros(M // p["BM"] + 1, N // p["BN"], device=cuda, dtype=torch.int32)
+    for tma in (-1, 0):
+        impl.set_option("tma_out", tma)
+        c = torch.full((M, N), float("nan"), device=cuda, dtype=dt)
+        impl.gemm_allreduce_overlap(a, b, c, mm, RA, rldn, e, e.to(cuda), algo, False)
+        ran = _ran(impl)
+        assert ran != (algo, 0, 0)
+        if M == 2560:
+            assert ran == (1, 0, 80 % (impl.get_option("sm_count") // 2))
+        _check(layout.from_reordered(c.cpu(), M, N, p["BM"], p["BN"], RA.cpu(), rldn).to(cuda), a, b, dt)
+    impl.set_option("tma_out", -1)
+    impl.check_status()
+
+
+def test_dependent_launches_across_streams(cuda, impl):
+    """The early launch waits for its own stream's predecessor and for what an event makes it wait for, and a
+    plain kernel behind it for all of it."""
+    dt = torch.bfloat16
+    M = N = K = 2048
+    a, b = (torch.randn(M, K, device=cuda).to(dt) for _ in range(2))
+    w = torch.ones(N, device=cuda, dtype=dt)
+    c, y, z, out = (torch.empty(M, N, device=cuda, dtype=dt) for _ in range(4))
+    side = torch.cuda.Stream()
+    main = torch.cuda.current_stream()
+    impl.cutlass_gemm(a, b, c, 1)
+    ref = ops.rmsnorm(c, w, 1e-5)
+    impl.cutlass_gemm(ref, b, z, 1)
+    expect = z + z
+    for _ in range(20):
+        for t in (c, y, z, out):
+            t.fill_(float("nan"))
+        impl.cutlass_gemm(a, b, c, 1)                             # main: writes c
+        done = torch.cuda.Event()
+        done.record()
+        with torch.cuda.stream(side):
+            side.wait_event(done)
+            torch.ops.flashoverlap_op.rmsnorm(c, y, w, 1e-5)      # side: behind the event
+            impl.cutlass_gemm(y, b, z, 1)                         # side: behind the norm, launched early
+            torch.add(z, z, out=out)
+            back = torch.cuda.Event()
+            back.record()
+        main.wait_event(back)
+        assert torch.equal(out, expect)
+    impl.check_status()
