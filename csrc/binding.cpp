@@ -81,7 +81,13 @@ void rmsnorm(at::Tensor X, at::Tensor RX, at::Tensor RW, double eps) {
 
 bool aligned16(const at::Tensor& t) { return reinterpret_cast<uintptr_t>(t.data_ptr()) % 16 == 0; }
 
-// H = X + T, RX = rmsnorm(H) * RW; H may be X.
+// Whether output `o` shares memory with `t` other than by being it (equal sizes): the row kernels read an
+// element and store it in the same thread.
+bool clashes(const at::Tensor& o, const at::Tensor& t) {
+  return o.data_ptr() != t.data_ptr() && fo::overlaps(o, o.numel(), t, t.numel());
+}
+
+// H = X + T, RX = rmsnorm(H) * RW; H and RX may be X or T, not the same one.
 void add_rmsnorm(at::Tensor X, at::Tensor T, at::Tensor H, at::Tensor RX, at::Tensor RW, double eps) {
   const bool bf = is_bf16(X, "X");
   is_bf16(T, "T");
@@ -94,7 +100,12 @@ void add_rmsnorm(at::Tensor X, at::Tensor T, at::Tensor H, at::Tensor RX, at::Te
   FO_CHECK(X.dim() == 2 && T.sizes() == X.sizes() && H.sizes() == X.sizes() && RX.sizes() == X.sizes(),
            "X, T, H and RX must be [rows, dim]");
   FO_CHECK(RW.numel() == X.size(1), "RW must have dim elements");
-  FO_CHECK(H.data_ptr() != RX.data_ptr() || X.numel() == 0, "H and RX must not alias");
+  for (const at::Tensor& t : {T, H, RX, RW}) fo::check_device(t, X, "an operand of add_rmsnorm");
+  FO_CHECK(!fo::overlaps(H, H.numel(), RX, RX.numel()), "H and RX must not alias");
+  FO_CHECK(!clashes(H, X) && !clashes(H, T) && !clashes(RX, X) && !clashes(RX, T),
+           "H and RX must each be X, T or memory of their own");
+  FO_CHECK(!fo::overlaps(RW, RW.numel(), H, H.numel()) && !fo::overlaps(RW, RW.numel(), RX, RX.numel()),
+           "RW must not alias H or RX");
   FO_CHECK(aligned16(X) && aligned16(T) && aligned16(H) && aligned16(RX) && aligned16(RW),
            "all tensors must be 16-byte aligned");
   c10::cuda::CUDAGuard guard(X.device());
@@ -128,6 +139,8 @@ void swiglu(at::Tensor GU, at::Tensor Y) {
            "GU must be [rows, 2 f] and Y [rows, f]");
   FO_CHECK(Y.size(1) % 8 == 0, "f must be a multiple of 8");
   FO_CHECK(aligned16(GU) && aligned16(Y), "GU and Y must be 16-byte aligned");
+  fo::check_device(Y, GU, "Y");
+  FO_CHECK(!fo::overlaps(Y, Y.numel(), GU, GU.numel()), "Y must not alias GU");
   c10::cuda::CUDAGuard guard(GU.device());
   fo::cuda_check(fo::swiglu_launch(GU.data_ptr(), Y.data_ptr(), static_cast<int>(GU.size(0)),
                                    static_cast<int>(Y.size(1)), bf, sm_count_of_current_device(),

@@ -55,6 +55,10 @@ inline void check_out(const at::Tensor& C, const at::Tensor& A, int64_t numel, c
   FO_CHECK(C.numel() >= numel, name, " is too small: needs ", numel, " elements");
 }
 
+inline void check_device(const at::Tensor& t, const at::Tensor& like, const char* name) {
+  FO_CHECK(t.device() == like.device(), name, " is on another device");
+}
+
 // Whether the first `a_numel` elements of `a` share memory with the first `b_numel` of `b`.
 inline bool overlaps(const at::Tensor& a, int64_t a_numel, const at::Tensor& b, int64_t b_numel) {
   const auto a0 = reinterpret_cast<uintptr_t>(a.data_ptr()), b0 = reinterpret_cast<uintptr_t>(b.data_ptr());

@@ -364,9 +364,13 @@ void OverlapImpl::Gemm(at::Tensor A, at::Tensor B, at::Tensor C, int64_t Algo) {
 
 void OverlapImpl::GemmAdd(at::Tensor A, at::Tensor B, at::Tensor R, at::Tensor C, int64_t Algo) {
   NvtxRange nvtx_range("flashoverlap::gemm_add");
+  FO_CHECK(world_ == 1, "gemm_add adds one rank's product: use gemm_reducescatter_add_rmsnorm_fused on several");
   const GemmShape s = check_operands(A, B);
   check_out(C, A, static_cast<int64_t>(s.M) * s.N, "C");
   check_out(R, A, static_cast<int64_t>(s.M) * s.N, "R");
+  check_device(B, A, "B");
+  check_device(R, A, "R");
+  check_device(C, A, "C");
   FO_CHECK(reinterpret_cast<uintptr_t>(R.data_ptr()) % 16 == 0, "R must be 16-byte aligned");
   const int64_t numel = static_cast<int64_t>(s.M) * s.N;
   FO_CHECK(!overlaps(C, numel, A, A.numel()) && !overlaps(C, numel, B, B.numel()), "C must not overlap A or B");
@@ -377,13 +381,16 @@ void OverlapImpl::GemmAdd(at::Tensor A, at::Tensor B, at::Tensor R, at::Tensor C
 
 void OverlapImpl::GemmSwiGLU(at::Tensor A, at::Tensor B, at::Tensor C) {
   NvtxRange nvtx_range("flashoverlap::gemm_swiglu");
+  FO_CHECK(world_ == 1, "gemm_swiglu is a single-rank call");
+  const GemmShape s = check_operands(A, B);
   if (heap_ == nullptr) NcclInit(0, 1, {});
   c10::cuda::CUDAGuard guard(A.device());
-  const GemmShape s = check_operands(A, B);
   const int f = s.N / 2;
   FO_CHECK(s.M % kBM == 0 && s.N % 256 == 0 && s.K % 8 == 0, "gemm_swiglu needs M a multiple of 128, ",
            "B of 2 * N rows with N a multiple of 128, and K a multiple of 8 (M=", s.M, " rows of B=", s.N, " K=", s.K, ")");
   check_out(C, A, static_cast<int64_t>(s.M) * f, "C");
+  check_device(B, A, "B");
+  check_device(C, A, "C");
   const int64_t numel = static_cast<int64_t>(s.M) * f;
   FO_CHECK(!overlaps(C, numel, A, A.numel()) && !overlaps(C, numel, B, B.numel()), "C must not overlap A or B");
   constexpr int kPairAlgo = 1;  // CTA pairs, 256-wide B tiles, strips of 8

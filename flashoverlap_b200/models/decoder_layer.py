@@ -175,10 +175,10 @@ class TPDecoderLayer(nn.Module):
         return self._rank_gemms(x.device) is not None
 
     def _rank_gemms(self, device: torch.device):
-        """The object whose GEMMs one rank runs: the caller's, or one of the layer's own, made with the layer (and
-        again on first use on another device).  None where it would have to be made while a stream
-        is being captured: its status words would belong to the graph."""
-        if self.ov is not None:
+        """The object whose GEMMs one rank runs: the caller's if it is a single-rank one, or one of the layer's own,
+        made with the layer (and again on first use on another device).  None where it would have to be
+        made while a stream is being captured: its status words would belong to the graph."""
+        if self.ov is not None and self.ov.get_option("world") == 1:
             return self.ov
         if self._one_rank is None or self._one_rank[0] != device:
             if torch.cuda.is_current_stream_capturing():

@@ -225,3 +225,54 @@ def test_layer_check_status_reports_a_wait_that_gave_up(cuda):
         layer.check_status()
     own.reset_status()
     layer.check_status()
+
+
+def test_add_rmsnorm_operands_in_place_or_apart(cuda):
+    mem = torch.randn(16, 64, device=cuda).to(torch.bfloat16)
+    x, t, w = mem[:4], mem[4:8], torch.ones(64, device=cuda, dtype=torch.bfloat16)
+    h, y = x + t, ops.rmsnorm(x + t, w, 1e-5)
+    for out, norm in ((mem[8:12], x), (t, mem[8:12]), (mem[8:12], t)):
+        keep = mem.clone()
+        _op().add_rmsnorm(x, t, out, norm, w, 1e-5)
+        assert torch.equal(out, h) and torch.equal(norm, y)
+        mem.copy_(keep)
+    for out, norm in ((mem[2:6], mem[8:12]), (mem[8:12], mem[5:9]), (mem[8:12], mem[8:12]), (mem[8:12], mem[10:14])):
+        with pytest.raises(RuntimeError):
+            _op().add_rmsnorm(x, t, out, norm, w, 1e-5)
+    with pytest.raises(RuntimeError):
+        _op().add_rmsnorm(x, t, mem[8:12], mem[12:16], mem[9], 1e-5)
+
+
+def test_rope_and_swiglu_refuse(cuda):
+    qkv = torch.zeros(4, 256, device=cuda, dtype=torch.bfloat16)
+    _op().rope_(qkv, 4, 2, 128, 1e4)
+    for bad, seq, heads, hd in ((qkv, 4, 3, 128), (qkv, 0, 2, 128), (qkv, 4, 2, 12), (qkv, 4, -1, 128), (qkv.float(), 4, 2, 128),
+                                (qkv[:, :128], 4, 1, 128), (qkv.view(-1), 4, 2, 128), (qkv.cpu(), 4, 2, 128),
+                                (qkv.view(-1)[4:1012].view(4, 252), 4, 1, 128)):
+        with pytest.raises(RuntimeError):
+            _op().rope_(bad, seq, heads, hd, 1e4)
+    gu, y = torch.zeros(4, 256, device=cuda, dtype=torch.bfloat16), torch.zeros(4, 128, device=cuda, dtype=torch.bfloat16)
+    _op().swiglu(gu, y)
+    for a, b in ((gu, y[:, :64]), (gu, y[:2]), (gu, y.half()), (gu.float(), y.float()), (gu, y.cpu()), (gu.view(-1), y), (gu[:, ::2], y),
+                 (gu[:, :24].contiguous(), y[:, :12].contiguous()), (gu, gu.view(-1)[:512].view(4, 128)), (gu, gu.view(-1)[512:].view(4, 128))):
+        with pytest.raises(RuntimeError):
+            _op().swiglu(a, b)
+
+
+def test_epilogue_gemms_refuse(cuda, impl):
+    a, b, r, c = (torch.zeros(256, 256, device=cuda, dtype=torch.bfloat16) for _ in range(4))
+    impl.gemm_add(a, b, r, c, 0)
+    for bad in ((a[:, :128], b, r, c), (a, b.half(), r, c), (a, b, r[:128], c), (a, b, r, c[:128]), (a, b, r.half(), c), (a, b, r, c.float()),
+                (a.cpu(), b, r, c), (a, b, r.cpu(), c), (a, b, r.t()[:, ::2], c), (a[:64], b, r, c)):
+        with pytest.raises(RuntimeError):
+            impl.gemm_add(*bad, 0)
+    for algo in (-1, 1000):
+        with pytest.raises(RuntimeError):
+            impl.gemm_add(a, b, r, c, algo)
+    y = torch.zeros(256, 128, device=cuda, dtype=torch.bfloat16)
+    impl.gemm_swiglu(a, b, y)
+    for bad in ((a[:64], b, y), (a, b[:128], y), (a, b, y[:64]), (a, b.half(), y), (a, b, y.half()), (a, b, y.cpu()), (a[:, :128], b, y),
+                (a[:, :4].contiguous(), b[:, :4].contiguous(), y)):
+        with pytest.raises(RuntimeError):
+            impl.gemm_swiglu(*bad)
+    impl.check_status()

@@ -487,3 +487,21 @@ def test_launch_skew_between_ranks(lib):
         assert r.pop("status") == 0
         for k, v in r.items():
             assert v <= 1.0, (k, v)
+
+
+def _single_rank_calls_worker(rank, world):
+    impl = _setup(rank, world)
+    dev = torch.device("cuda", rank)
+    a, b, r = (torch.zeros(256, 256, device=dev, dtype=torch.bfloat16) for _ in range(3))
+    refused = 0
+    for call in (lambda: impl.gemm_add(a, b, r, r, 0), lambda: impl.gemm_swiglu(a, b, torch.empty_like(r))):
+        try:
+            call()
+        except RuntimeError:
+            refused += 1
+    return refused
+
+
+def test_single_rank_gemms_are_refused_on_several_ranks(lib):
+    """They would return this rank's unreduced product."""
+    assert list(run_ranks(_single_rank_calls_worker, _world(), "nccl")) == [2] * _world()
