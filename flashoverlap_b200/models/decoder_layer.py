@@ -25,6 +25,7 @@ import torch
 import torch.distributed as dist
 import torch.nn as nn
 import torch.nn.functional as F
+from torch.autograd import forward_ad
 
 from ..utils import config, layout
 
@@ -55,6 +56,12 @@ class DecoderConfig:
     @staticmethod
     def tiny() -> "DecoderConfig":
         return DecoderConfig(hidden=1024, ffn=2048, n_heads=8, n_kv_heads=2, head_dim=128)
+
+
+def _transforming() -> bool:
+    """Inside a function transform (vmap, jvp, ...), a forward-mode level or a trace."""
+    return (torch._C._functorch.peek_interpreter_stack() is not None or forward_ad._current_level >= 0
+            or torch._C._is_tracing())
 
 
 def _rope(x: torch.Tensor, theta: float) -> torch.Tensor:
@@ -133,10 +140,11 @@ class TPDecoderLayer(nn.Module):
 
     @staticmethod
     def _native(t: torch.Tensor) -> bool:
-        """Whether the fused element-wise kernels take ``t``: 16-bit, contiguous, on a GPU, and no
-        autograd graph to record (they have no backward)."""
-        if not (t.is_cuda and t.dtype in (torch.bfloat16, torch.float16) and t.is_contiguous()
-                and t.data_ptr() % 16 == 0) or (torch.is_grad_enabled() and t.requires_grad):
+        """Whether the fused element-wise kernels take ``t``: 16-bit, contiguous, on a GPU, and nothing that
+        only torch's own operators do is asked of it - a graph to record, a tangent to carry along, a
+        function transform (vmap, jvp), a trace."""
+        if not (t.is_cuda and t.dtype in (torch.bfloat16, torch.float16) and t.is_contiguous()) or \
+                (t.requires_grad and torch.is_grad_enabled()) or _transforming() or t.data_ptr() % 16:
             return False
         from .._build import load
         load()

@@ -276,3 +276,24 @@ def test_epilogue_gemms_refuse(cuda, impl):
         with pytest.raises(RuntimeError):
             impl.gemm_swiglu(*bad)
     impl.check_status()
+
+
+def test_one_rank_layer_under_function_transforms(cuda):
+    """vmap and forward mode over weights, which the fused kernels know nothing of, reach torch's operators."""
+    from torch.autograd import forward_ad
+    layer, x = _one_rank_layer(cuda)
+    call = lambda **weights: torch.func.functional_call(layer, weights, (x,))
+    wd = torch.stack([layer.wd.detach(), 2 * layer.wd.detach()])
+    wgu = torch.stack([layer.wgu.detach(), layer.wgu.detach().flip(0)])
+    with torch.no_grad():
+        for name, many in (("wd", wd), ("wgu", wgu)):
+            got = torch.vmap(lambda w: call(**{name: w}))(many)
+            for i in range(2):
+                ref = call(**{name: many[i]})
+                assert (got[i] - ref).abs().max() <= 2.0 ** -6 * ref.abs().max()     # they round at different places
+        tangent = torch.randn_like(layer.wd)
+        with forward_ad.dual_level():
+            out = forward_ad.unpack_dual(call(wd=forward_ad.make_dual(layer.wd.detach(), tangent)))
+        # the output is linear in wd: its tangent is what the layer adds for the tangent's weights
+        step = call(wd=tangent).float() - call(wd=torch.zeros_like(tangent)).float()
+        assert out.tangent is not None and (out.tangent.float() - step).abs().max() <= 2.0 ** -6 * step.abs().max()
