@@ -290,8 +290,13 @@ void OverlapImpl::run_plain(const at::Tensor& A, const at::Tensor& B, void* out,
   GemmTensorMaps maps;
   GemmParams p;
   std::memset(&p, 0, sizeof(p));
-  bool bf16 = true;
-  setup_problem(algo, A, B, 0, &maps, &p, &bf16);
+  const GemmShape s = check_operands(A, B);
+  const bool bf16 = s.bf16;
+  p.M = s.M;
+  p.N = s.N;
+  p.K = s.K;
+  std::string e = prepare_tiling(algo, &p);
+  FO_CHECK(e.empty(), e, " (M=", s.M, " N=", s.N, " K=", s.K, " Algo=", algo, ")");
   p.out_mode = out_mode;
   p.rldn = rldn < 1 ? 1 : rldn;
   p.signal = signal ? 1 : 0;
@@ -318,12 +323,11 @@ void OverlapImpl::run_plain(const at::Tensor& A, const at::Tensor& B, void* out,
   last_tail_ = 0;
   const AlgoConfig c = algo_config(plan.algo);
   const int bn = plan.split != 0 ? kSplitBN : c.bn;
-  const int b_rows = plan.split == 0 && c.cta2 ? bn / 2 : bn;
-  const AlgoConfig own = algo_config(algo);
-  if (b_rows != (own.cta2 ? own.bn / 2 : own.bn)) {
-    const std::string e = encode_tmap_16bit(&maps.b[0], B.data_ptr(), p.N, p.K, b_rows);
-    FO_CHECK(e.empty(), "B: ", e);
-  }
+  // each map once, for the kernel that runs
+  e = encode_tmap_16bit(&maps.a[0], A.data_ptr(), p.M, p.K, kBM);
+  FO_CHECK(e.empty(), "A: ", e);
+  e = encode_tmap_16bit(&maps.b[0], B.data_ptr(), p.N, p.K, plan.split == 0 && c.cta2 ? bn / 2 : bn);
+  FO_CHECK(e.empty(), "B: ", e);
   p.tiles_n = p.N / bn;
   set_raster(c.raster_sw, &p);
   set_l2_hints(&p, opt_l2_hints_ != 0);
@@ -347,7 +351,7 @@ void OverlapImpl::run_plain(const at::Tensor& A, const at::Tensor& B, void* out,
     if (tail > 0) {
       p.tail_start = units - tail;
       last_tail_ = tail;
-      const std::string e = encode_tmap_16bit(&maps.b[1], B.data_ptr(), p.N, p.K, bn / 4);
+      e = encode_tmap_16bit(&maps.b[1], B.data_ptr(), p.N, p.K, bn / 4);
       FO_CHECK(e.empty(), "B: ", e);
     }
   }
