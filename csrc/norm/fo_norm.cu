@@ -482,9 +482,15 @@ cudaError_t launch_norm(const void* X, void* Y, const void* W, int rows, int dim
 
 }  // namespace
 
+// Every tensor here is read and written 16 bytes at a time.
+template <typename... P>
+static bool unaligned(P... p) {
+  return ((reinterpret_cast<uintptr_t>(p) | ...) & 15) != 0;
+}
+
 cudaError_t rmsnorm_launch(const void* X, void* Y, const void* W, int rows, int dim, float eps,
                            bool bf16, int sm_count, cudaStream_t stream) {
-  if (dim % 8 != 0) return cudaErrorInvalidValue;
+  if (dim % 8 != 0 || (rows > 0 && unaligned(X, Y, W))) return cudaErrorInvalidValue;
   if (rows == 0) return cudaSuccess;
   return bf16 ? launch_norm<true, false>(X, Y, W, rows, dim, 1, 1, 1, nullptr, eps, sm_count, stream)
               : launch_norm<false, false>(X, Y, W, rows, dim, 1, 1, 1, nullptr, eps, sm_count, stream);
@@ -492,7 +498,7 @@ cudaError_t rmsnorm_launch(const void* X, void* Y, const void* W, int rows, int 
 
 cudaError_t add_rmsnorm_launch(const void* X, const void* T, void* H, void* Y, const void* W, int rows, int dim,
                                float eps, bool bf16, int sm_count, cudaStream_t stream) {
-  if (dim % 8 != 0) return cudaErrorInvalidValue;
+  if (dim % 8 != 0 || (rows > 0 && unaligned(X, T, H, Y, W))) return cudaErrorInvalidValue;
   if (rows == 0) return cudaSuccess;
   return bf16 ? launch_add_norm<true>(X, T, H, Y, W, rows, dim, eps, sm_count, stream)
               : launch_add_norm<false>(X, T, H, Y, W, rows, dim, eps, sm_count, stream);
@@ -501,7 +507,8 @@ cudaError_t add_rmsnorm_launch(const void* X, const void* T, void* H, void* Y, c
 cudaError_t reorder_rmsnorm_launch(const void* X, void* Y, const void* W, int rows, int dim, int BM,
                                    int BN, int rldn, const int* RA, float eps, bool bf16,
                                    int sm_count, cudaStream_t stream) {
-  if (dim % 8 != 0 || BN % 8 != 0 || dim % BN != 0 || rows % BM != 0 || rldn < 1)
+  if (dim % 8 != 0 || BN % 8 != 0 || dim % BN != 0 || rows % BM != 0 || rldn < 1 ||
+      (rows > 0 && unaligned(X, Y, W)))
     return cudaErrorInvalidValue;
   if (rows == 0) return cudaSuccess;
   return bf16 ? launch_norm<true, true>(X, Y, W, rows, dim, BM, BN, rldn, RA, eps, sm_count, stream)
@@ -510,7 +517,8 @@ cudaError_t reorder_rmsnorm_launch(const void* X, void* Y, const void* W, int ro
 
 cudaError_t reorder_launch(const void* X, void* Y, int rows, int dim, int BM, int BN, int rldn,
                            const int* RA, bool to_reordered, int sm_count, cudaStream_t stream) {
-  if (dim % 8 != 0 || BN % 8 != 0 || dim % BN != 0 || rows % BM != 0 || rldn < 1)
+  if (dim % 8 != 0 || BN % 8 != 0 || dim % BN != 0 || rows % BM != 0 || rldn < 1 ||
+      (rows > 0 && unaligned(X, Y)))
     return cudaErrorInvalidValue;
   if (rows == 0) return cudaSuccess;
   const int nvec = dim / 8;

@@ -55,6 +55,11 @@ inline void check_out(const at::Tensor& C, const at::Tensor& A, int64_t numel, c
   FO_CHECK(C.numel() >= numel, name, " is too small: needs ", numel, " elements");
 }
 
+// The kernels store 16 bytes at a time: refused here, an unaligned output would fault there.
+inline void check_aligned(const void* p, const char* name) {
+  FO_CHECK(reinterpret_cast<uintptr_t>(p) % 16 == 0, name, " must be 16-byte aligned");
+}
+
 inline void check_device(const at::Tensor& t, const at::Tensor& like, const char* name) {
   FO_CHECK(t.device() == like.device(), name, " is on another device");
 }

@@ -142,6 +142,7 @@ std::vector<int64_t> fused_loopback(std::string comm_op, std::vector<at::Tensor>
       FO_CHECK(static_cast<int>(norm_res->size()) == ws, "norm_res needs one tensor per rank");
       for (int r = 0; r < ws; ++r) {
         check_out((*norm_res)[r], A[0], shard, "norm_res");
+        check_aligned((*norm_res)[r].data_ptr(), "norm_res");
         p.norm_res[r] = (*norm_res)[r].data_ptr();
       }
     }
@@ -149,6 +150,7 @@ std::vector<int64_t> fused_loopback(std::string comm_op, std::vector<at::Tensor>
       FO_CHECK(static_cast<int>(norm_out->size()) == ws, "norm_out needs one tensor per rank");
       for (int r = 0; r < ws; ++r) {
         check_out((*norm_out)[r], A[0], shard, "norm_out");
+        check_aligned((*norm_out)[r].data_ptr(), "norm_out");
         p.norm_out[r] = (*norm_out)[r].data_ptr();
       }
     }
@@ -170,6 +172,7 @@ std::vector<int64_t> fused_loopback(std::string comm_op, std::vector<at::Tensor>
     p.flags[r] = reinterpret_cast<uint32_t*>(sig + kSignalFlagsOffset);
     p.done[r] = reinterpret_cast<uint32_t*>(sig + kSignalDoneOffset);
     p.ready[r] = reinterpret_cast<uint32_t*>(sig + kSignalReadyOffset);
+    check_aligned(out[r].data_ptr(), "out");
     p.dst[r] = out[r].data_ptr();
   }
   const int per_rank = std::max(1, std::min(sm_count / ws, p.num_tiles));

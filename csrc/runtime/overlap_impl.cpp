@@ -313,6 +313,7 @@ void OverlapImpl::run_plain(const at::Tensor& A, const at::Tensor& B, void* out,
   p.cseg = cseg;
   p.out[0] = out;
   p.MM[0] = MM;
+  check_aligned(out, "the output");
   p.status[0] = status_.data_ptr<int>();
   p.epilogue = res != nullptr ? kEpiResidual : kEpiStore;
   p.res = res;
@@ -375,7 +376,7 @@ void OverlapImpl::GemmAdd(at::Tensor A, at::Tensor B, at::Tensor R, at::Tensor C
   check_device(B, A, "B");
   check_device(R, A, "R");
   check_device(C, A, "C");
-  FO_CHECK(reinterpret_cast<uintptr_t>(R.data_ptr()) % 16 == 0, "R must be 16-byte aligned");
+  check_aligned(R.data_ptr(), "R");
   const int64_t numel = static_cast<int64_t>(s.M) * s.N;
   FO_CHECK(!overlaps(C, numel, A, A.numel()) && !overlaps(C, numel, B, B.numel()), "C must not overlap A or B");
   FO_CHECK(C.data_ptr() == R.data_ptr() || !overlaps(C, numel, R, numel), "C must be R or not overlap it");
@@ -601,6 +602,7 @@ void OverlapImpl::run_fused(int comm, const at::Tensor& A, const at::Tensor& B, 
   } else {
     p.dst[rank_] = out.data_ptr();
   }
+  if (!copy_back) check_aligned(out.data_ptr(), "the output");
 
   // The call number enters the kernel's handshakes; it is advanced only once nothing can
   // reject the call any more (directly before the launch, and taken back if the launch fails):
@@ -641,11 +643,13 @@ void OverlapImpl::run_fused(int comm, const at::Tensor& A, const at::Tensor& B, 
     p.norm_eps = static_cast<float>(norm_eps);
     if (norm_res != nullptr) {
       check_out(*norm_res, A, static_cast<int64_t>(out_bytes / 2), "R");
+      check_aligned(norm_res->data_ptr(), "R");
       p.norm_res[rank_] = norm_res->data_ptr();
     }
     if (norm_out != nullptr) {
       check_out(*norm_out, A, static_cast<int64_t>(out_bytes / 2), "Y");
       FO_CHECK(norm_out->data_ptr() != out.data_ptr(), "Y must not alias the residual stream");
+      check_aligned(norm_out->data_ptr(), "Y");
       p.norm_out[rank_] = norm_out->data_ptr();
     }
     p.row_ssq = norm_ssq_.data_ptr<float>();

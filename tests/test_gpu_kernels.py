@@ -594,6 +594,27 @@ def test_row_parallel_layer_runs_a_timed_algo_as_it_was_timed(cuda):
     layer.overlap_class.check_status()
 
 
+def test_unaligned_tensors_are_refused(cuda):
+    """Whole rows are read and stored 16 bytes at a time; a view that starts in between is refused on the host."""
+    n = 256 * 256
+    mem = torch.zeros(n + 8, device=cuda, dtype=torch.bfloat16)
+    off = mem[4:4 + n].view(256, 256)
+    ok, w = torch.zeros(256, 256, device=cuda, dtype=torch.bfloat16), torch.ones(256, device=cuda, dtype=torch.bfloat16)
+    ra = torch.arange(2, device=cuda, dtype=torch.int32)
+    impl = ops.OverlapImpl()
+    impl.nccl_init(0, 1, [0] * 16)
+    raw = torch.ops.flashoverlap_op
+    for call in (lambda: raw.rmsnorm(off, ok, w, 1e-5), lambda: raw.rmsnorm(ok, off, w, 1e-5), lambda: raw.rmsnorm(ok, ok, mem[4:260], 1e-5),
+                 lambda: raw.reorder_rmsnorm_eps(off, ok, w, 128, 256, 1, ra, 1e-5),
+                 lambda: raw.reorder(off, ok, 128, 256, 1, ra), lambda: raw.unreorder(ok, off, 128, 256, 1, ra),
+                 lambda: impl.cutlass_gemm(ok, ok, off, 0), lambda: impl.cutlass_gemm(off, ok, ok.clone(), 0),
+                 lambda: impl.gemm_reducescatter_fused(ok, ok, off, 0),
+                 lambda: ops.fused_loopback("all_reduce", [ok, ok], [ok, ok], [ok.clone(), off])):
+        with pytest.raises(RuntimeError):
+            call()
+    torch.cuda.synchronize()
+
+
 # both builds of the kernel and every way its rows are dealt out, on either side of where they change: rows that one
 # and two waves hold, the last wave nearly full and not, one wave of many narrow rows; 1, 2, 4 and 8 vectors a thread
 @pytest.mark.parametrize("dim,BN,rows", [(256, 256, (16, 880, 896, 1040, 1792, 2064, 2080, 2944, 2960, 5696, 9568, 16384)),
