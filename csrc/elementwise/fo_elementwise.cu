@@ -1,33 +1,14 @@
 #include "fo_elementwise.h"
 
-#include <cuda_bf16.h>
-#include <cuda_fp16.h>
 #include <cstdint>
+
+#include "../common/fo_pack16.cuh"
 
 namespace fo {
 
 namespace {
 
 constexpr int kThreads = 256;
-
-template <bool BF16>
-__device__ __forceinline__ float2 unpack(uint32_t w) {
-  if constexpr (BF16) {
-    return __bfloat1622float2(*reinterpret_cast<__nv_bfloat162*>(&w));
-  } else {
-    return __half22float2(*reinterpret_cast<__half2*>(&w));
-  }
-}
-template <bool BF16>
-__device__ __forceinline__ uint32_t pack(float a, float b) {
-  if constexpr (BF16) {
-    __nv_bfloat162 v = __floats2bfloat162_rn(a, b);
-    return *reinterpret_cast<uint32_t*>(&v);
-  } else {
-    __half2 v = __floats2half2_rn(a, b);
-    return *reinterpret_cast<uint32_t*>(&v);
-  }
-}
 
 // Bound by memory: 4096 tokens x 9 heads of 128 (19 MB moved) took 284 us as the fourteen eager
 // operators of the two rotations (fp32 intermediates, strided pairs) and take 9 us here.
@@ -64,8 +45,8 @@ __global__ void __launch_bounds__(kThreads)
       uint32_t* u = reinterpret_cast<uint32_t*>(&x[i]);
 #pragma unroll
       for (int k = 0; k < 4; ++k) {
-        const float2 v = unpack<BF16>(u[k]);
-        u[k] = pack<BF16>(v.x * c[k] - v.y * s[k], v.x * s[k] + v.y * c[k]);
+        const float2 v = unpack2<BF16>(u[k]);
+        u[k] = pack2<BF16>(v.x * c[k] - v.y * s[k], v.x * s[k] + v.y * c[k]);
       }
       *reinterpret_cast<uint4*>(row + static_cast<int64_t>(h0 + i) * head_dim) = x[i];
     }
@@ -74,11 +55,11 @@ __global__ void __launch_bounds__(kThreads)
 
 template <bool BF16>
 __device__ __forceinline__ uint32_t silu_mul(uint32_t g, uint32_t u) {
-  const float2 a = unpack<BF16>(g);
+  const float2 a = unpack2<BF16>(g);
   // silu is rounded to the storage type before the product, as two operators in a row round it
-  const uint32_t r = pack<BF16>(a.x / (1.f + expf(-a.x)), a.y / (1.f + expf(-a.y)));
-  const float2 p = unpack<BF16>(r), q = unpack<BF16>(u);
-  return pack<BF16>(p.x * q.x, p.y * q.y);
+  const uint32_t r = pack2<BF16>(silu(a.x), silu(a.y));
+  const float2 p = unpack2<BF16>(r), q = unpack2<BF16>(u);
+  return pack2<BF16>(p.x * q.x, p.y * q.y);
 }
 
 template <bool BF16>

@@ -1,9 +1,10 @@
-// Device helpers shared by the tcgen05 GEMM kernels: tile order, wave groups, 16-bit arithmetic.
+// Device helpers shared by the tcgen05 GEMM kernels: tile order, wave groups.
 #pragma once
 #include <cuda.h>
 #include <cuda_runtime.h>
 #include <cstdint>
 
+#include "../common/fo_pack16.cuh"
 #include "../common/fo_ptx.cuh"
 #include "fo_gemm_params.h"
 
@@ -60,38 +61,10 @@ __device__ __forceinline__ int tile_position(const GemmParams& p, int t, int32_t
 }
 
 template <bool BF16>
-__device__ __forceinline__ uint32_t pack2(float lo, float hi) {
-  if constexpr (BF16) {
-    __nv_bfloat162 v = __floats2bfloat162_rn(lo, hi);
-    return *reinterpret_cast<uint32_t*>(&v);
-  } else {
-    __half2 v = __floats2half2_rn(lo, hi);
-    return *reinterpret_cast<uint32_t*>(&v);
-  }
-}
-
-template <bool BF16>
 __device__ __forceinline__ void unpack_add(uint32_t w, float& lo, float& hi) {
-  if constexpr (BF16) {
-    __nv_bfloat162 v = *reinterpret_cast<__nv_bfloat162*>(&w);
-    float2 f = __bfloat1622float2(v);
-    lo += f.x;
-    hi += f.y;
-  } else {
-    __half2 v = *reinterpret_cast<__half2*>(&w);
-    float2 f = __half22float2(v);
-    lo += f.x;
-    hi += f.y;
-  }
-}
-
-// round16(a + b) per 16-bit pair, added in fp32: what `a + b` on 16-bit tensors computes.
-template <bool BF16>
-__device__ __forceinline__ uint32_t add2(uint32_t a, uint32_t b) {
-  float lo = 0.f, hi = 0.f;
-  unpack_add<BF16>(a, lo, hi);
-  unpack_add<BF16>(b, lo, hi);
-  return pack2<BF16>(lo, hi);
+  const float2 f = unpack2<BF16>(w);
+  lo += f.x;
+  hi += f.y;
 }
 
 }  // namespace fo

@@ -73,9 +73,10 @@ __device__ __forceinline__ uint4 add8(const uint4& a, const uint4& b) {
   return make_uint4(add2<BF16>(a.x, b.x), add2<BF16>(a.y, b.y), add2<BF16>(a.z, b.z), add2<BF16>(a.w, b.w));
 }
 
+// On the fp32 accumulators: nothing is rounded before the product is (the element-wise kernel, which reads
+// gate and up in 16 bits, also rounds silu, as two operators in a row do).
 __device__ __forceinline__ float silu_mul(uint32_t g, uint32_t u) {
-  const float x = __uint_as_float(g);
-  return x / (1.f + expf(-x)) * __uint_as_float(u);
+  return silu(__uint_as_float(g)) * __uint_as_float(u);
 }
 
 template <int BN, int STAGES, bool BF16, bool CTA2, int MT, int EPI>

@@ -10,10 +10,9 @@
 // thread keeps several 16-byte vectors in flight so that a B200 SM can cover HBM3e latency.
 #include "fo_norm.h"
 
-#include <cuda_bf16.h>
-#include <cuda_fp16.h>
 #include <cstdint>
 
+#include "../common/fo_pack16.cuh"
 #include "../common/fo_ptx.cuh"
 
 namespace fo {
@@ -21,15 +20,6 @@ namespace fo {
 namespace {
 
 constexpr int kNormThreads = 256;
-
-template <bool BF16>
-__device__ __forceinline__ float2 unpack2(uint32_t w) {
-  if constexpr (BF16) {
-    return __bfloat1622float2(*reinterpret_cast<__nv_bfloat162*>(&w));
-  } else {
-    return __half22float2(*reinterpret_cast<__half2*>(&w));
-  }
-}
 
 // y = round16(round16(x * scale) * w): the normalised value is rounded to the storage type
 // before the weight multiply, as in the reference (src/rmsnorm/rmsnorm.cuh:108-113) and in
@@ -44,19 +34,6 @@ __device__ __forceinline__ uint32_t scale_mul2(uint32_t x, uint32_t w, float sca
   } else {
     __half2 n = __floats2half2_rn(xf.x * scale, xf.y * scale);
     __half2 r = __hmul2(n, *reinterpret_cast<__half2*>(&w));
-    return *reinterpret_cast<uint32_t*>(&r);
-  }
-}
-
-// round16(a + b) per 16-bit pair, added in fp32: what `a + b` on 16-bit tensors computes.
-template <bool BF16>
-__device__ __forceinline__ uint32_t add2_16(uint32_t a, uint32_t b) {
-  const float2 x = unpack2<BF16>(a), y = unpack2<BF16>(b);
-  if constexpr (BF16) {
-    __nv_bfloat162 r = __floats2bfloat162_rn(x.x + y.x, x.y + y.y);
-    return *reinterpret_cast<uint32_t*>(&r);
-  } else {
-    __half2 r = __floats2half2_rn(x.x + y.x, x.y + y.y);
     return *reinterpret_cast<uint32_t*>(&r);
   }
 }
@@ -244,8 +221,8 @@ __global__ void __launch_bounds__(kNormThreads, (VPT <= 2 ? 4 : 2))
     for (int i = 0; i < VPT; ++i) {
       const int j = threadIdx.x + i * kNormThreads;
       if (j < nvec) {
-        h[i] = make_uint4(add2_16<BF16>(x[i].x, t[i].x), add2_16<BF16>(x[i].y, t[i].y),
-                          add2_16<BF16>(x[i].z, t[i].z), add2_16<BF16>(x[i].w, t[i].w));
+        h[i] = make_uint4(add2<BF16>(x[i].x, t[i].x), add2<BF16>(x[i].y, t[i].y),
+                          add2<BF16>(x[i].z, t[i].z), add2<BF16>(x[i].w, t[i].w));
         const uint32_t* u = reinterpret_cast<const uint32_t*>(&h[i]);
 #pragma unroll
         for (int k = 0; k < 4; ++k) {
