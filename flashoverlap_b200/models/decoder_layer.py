@@ -30,13 +30,17 @@ from torch.autograd import forward_ad
 from ..utils import config, layout
 
 TILE_M = 128
-# From these sizes on one rank's GEMMs take the residual (output elements) and SwiGLU (tokens) into their
-# epilogue.  Below them the library's small-problem kernels make up for the extra pass, e.g. 9.1 us
-# against 8.3 us for 1024 x 1024 x 2048 + residual and 94 against 89 us for SwiGLU of 1024 tokens, hidden 8192, ffn
-# 3584; above, 24.7 against 26.0 us for 1024 x 4096 x 3584 + residual, 158 against 214 us for 4096 x 8192 x 3584 +
-# residual, 157 against 188 us for SwiGLU of 4096 tokens, hidden 4096.
-MIN_ADD_ELEMENTS = 4 * 1024 * 1024
-MIN_SWIGLU_TOKENS = 2048
+# Where one rank's GEMMs take the residual and SwiGLU into their epilogue.  The alternative is the library's product
+# and one element-wise kernel; measured on a B200, in us a call, library against epilogue:
+# * SwiGLU from 2048 tokens on, if the GEMM's units of 256 tokens x 128 columns nearly fill the 74 CTA pairs once:
+#   2048 tokens, hidden 4096: 19.5 / 27.8 at ffn 512 (32 units), 30.3 / 29.0 at 1024 (64), 93 / 83 at 3584 (224); hidden 1024:
+#   24.2 / 23.6 at ffn 1024, 39.2 / 34.3 at 2048.  Below 2048 tokens it is even: 1024 x 8192 x 3584 89 / 93, 1024 x 4096 x 3584 50 / 48.
+# * The residual from 16 M output elements on, and from 4 M on unless K is long, where the library's main
+#   loop makes up for the extra pass: 2048 x 4096 x 3584 47.3 / 43.9, x 7168 85 / 86, x 14336 164 / 169; 4096 x 4096 x 14336 338 / 316.
+#   With the norm behind it (the library's side then adds in the norm's pass) also not for little work on narrow rows:
+#   2048 x 2048 x 512 12.7 / 13.3, x 2048 21.5 / 20.8; 4096 x 2048 x 512 20.4 / 18.7; 1024 x 4096 x 512 12.2 / 12.2.
+MIN_SWIGLU_TOKENS, MIN_SWIGLU_UNITS = 2048, 64
+MIN_ADD_ELEMENTS, ALWAYS_ADD_ELEMENTS, MAX_ADD_K = 4 << 20, 16 << 20, 4096
 
 
 @dataclass
@@ -208,10 +212,23 @@ class TPDecoderLayer(nn.Module):
     def __getstate__(self):
         return {**self.__dict__, "_one_rank": None}      # copies and files of the layer make their own
 
-    def _adds(self, x_sp, x, weight) -> bool:
-        """Whether the row-parallel projection of ``x`` adds the residual in its epilogue."""
-        return (x_sp.numel() >= MIN_ADD_ELEMENTS and x_sp.dtype == x.dtype
-                and x_sp.shape == (x.shape[0], weight.shape[0]) and self._fused_gemm(x, weight, x_sp))
+    def _adds(self, x_sp, x, weight, norm: bool = False) -> bool:
+        """Whether the row-parallel projection of ``x`` adds the residual in its epilogue; ``norm``: with the
+        norm of the sum behind it."""
+        n, k = x_sp.numel(), x.shape[1]
+        if n < ALWAYS_ADD_ELEMENTS:
+            if n < MIN_ADD_ELEMENTS or k > MAX_ADD_K:
+                return False
+            if norm and n < 2 * MIN_ADD_ELEMENTS and k < 2048 and x_sp.shape[-1] < 4096:
+                return False
+        return (x_sp.dtype == x.dtype and x_sp.shape == (x.shape[0], weight.shape[0])
+                and self._fused_gemm(x, weight, x_sp))
+
+    def _swiglus(self, hn) -> bool:
+        """Whether the gate and up projections of ``hn`` multiply in their epilogue."""
+        tokens, f = hn.shape[0], self.ffn_local
+        return (tokens >= MIN_SWIGLU_TOKENS and f % 128 == 0 and -(-tokens // 256) * (f // 128) >= MIN_SWIGLU_UNITS
+                and self._fused_gemm(hn, self.wgu))
 
     def _add_row_parallel(self, x_sp: torch.Tensor, x: torch.Tensor, weight: torch.Tensor) -> torch.Tensor:
         """``x_sp`` + the row-parallel projection of ``x``."""
@@ -269,14 +286,14 @@ class TPDecoderLayer(nn.Module):
                                                          cfg.eps, self.algo)
             hn = self._all_gather_tokens(hn_sp)
         else:
-            if self._adds(x_sp, attn, self.wo):
+            if self._adds(x_sp, attn, self.wo, norm=True):
                 h_sp = self._add_row_parallel(x_sp, attn, self.wo)             # [T/tp, h]
                 hn_sp = self._norm(h_sp, self.mlp_norm)
             else:
                 h_sp, hn_sp = self._add_norm(x_sp, self._row_parallel(attn, self.wo), self.mlp_norm)
             hn = self._all_gather_tokens(hn_sp)
         # MLP block
-        if hn.shape[0] >= MIN_SWIGLU_TOKENS and self.ffn_local % 128 == 0 and self._fused_gemm(hn, self.wgu):
+        if self._swiglus(hn):
             act = torch.empty((B * S, self.ffn_local), dtype=hn.dtype, device=hn.device)
             self._rank_gemms(hn.device).gemm_swiglu(hn, self.wgu, act)
             return self._add_row_parallel(h_sp, act, self.wd)

@@ -297,3 +297,23 @@ def test_one_rank_layer_under_function_transforms(cuda):
         # the output is linear in wd: its tangent is what the layer adds for the tangent's weights
         step = call(wd=tangent).float() - call(wd=torch.zeros_like(tangent)).float()
         assert out.tangent is not None and (out.tangent.float() - step).abs().max() <= 2.0 ** -6 * step.abs().max()
+
+
+@pytest.mark.parametrize("T,hidden,ffn,adds,swiglus", [
+    (2048, 2048, 512, (False, True), False), (2048, 2048, 1024, (False, True), True), (1920, 2048, 4096, (False, False), False),
+    (2048, 4096, 2048, (True, True), True), (2048, 2048, 5120, (False, False), True), (2048, 8192, 5120, (True, True), True)])
+def test_one_rank_layer_epilogues_by_size(cuda, T, hidden, ffn, adds, swiglus):
+    """What the layer leaves to its GEMMs' epilogues, and that it computes the same either way."""
+    from flashoverlap_b200.models import DecoderConfig, TPDecoderLayer
+    cfg = DecoderConfig(hidden=hidden, ffn=ffn, n_heads=4, n_kv_heads=2)
+    layer = TPDecoderLayer(cfg, 0, 1, 1, T, impl="fused", device=cuda)
+    x = torch.randn(T, hidden, device=cuda).to(torch.bfloat16)
+    with torch.no_grad():
+        attn, act = x[:, :512].contiguous(), torch.randn(T, ffn, device=cuda).to(torch.bfloat16)
+        assert (layer._adds(x, attn, layer.wo, norm=True), layer._adds(x, act, layer.wd)) == adds
+        assert layer._swiglus(x) == swiglus
+        y = layer(x)
+        layer._fused_gemm = lambda *_: False
+        plain = layer(x)
+    assert (y - plain).abs().max() <= 2.0 ** -6 * plain.abs().max()       # they round at different places
+    layer.check_status()
