@@ -541,6 +541,7 @@ __global__ void __launch_bounds__(kPlainThreads, 1)
     if (use_tma && lane == 0) ptx::bulk_wait_group<0>();
   }
 
+  __syncwarp();  // lanes that drained join theirs: the barriers' aligned forms take whole warps
   ptx::tc_fence_before_sync();
   if constexpr (CTA2) {
     // Neither CTA may free TMEM or leave while the other can still signal its barriers or

@@ -190,6 +190,7 @@ __global__ void __launch_bounds__(kSplitThreads, 1)
       ptx::report_status(status, kStatusTimeoutTmemFull, pos, 0, 0);
       *s_abort = 1;
     }
+    __syncwarp();  // the barrier's aligned form takes whole warps
     ptx::tc_fence_after_sync();
     ptx::cluster_wait_acquire();
     if (ok) {
@@ -218,6 +219,7 @@ __global__ void __launch_bounds__(kSplitThreads, 1)
       ptx::st_shared_cluster_u32(ptx::mapa_shared(ptx::smem_u32(misc + 2), lane), 1u);
     }
   }
+  __syncwarp();
   if (warp_idx < 2) ptx::cluster_wait_acquire();
 
   // Every CTA's partial sums have arrived (release / acquire at cluster scope).

@@ -39,3 +39,12 @@ def test_objects_and_launches_query_no_device_properties():
     """cudaGetDeviceProperties takes milliseconds: not once per object, nor per kernel of a choice."""
     for path in ("runtime/overlap_impl.cpp", "runtime/loopback.cpp", "gemm/fo_gemm_launch.cuh", "gemm/fo_gemm_splitk_launch.cu"):
         assert "cudaGetDeviceProperties(" not in re.sub(r"//[^\n]*", "", (GEMM.parent / path).read_text()), path
+
+
+@pytest.mark.parametrize("name,barrier", [("fo_gemm_plain_sm100.cuh", "cluster_arrive_relaxed"), ("fo_gemm_splitk_sm100.cuh", "cluster_arrive_release")])
+def test_roles_join_their_warps_before_the_cluster_barrier(name, barrier):
+    """barrier.cluster's aligned form is undefined for a warp whose lanes arrive apart; the roles end in
+    code that one lane runs."""
+    code = _code(name)
+    tail = code[:code.rindex(barrier)].rstrip()
+    assert "__syncwarp();" in tail[-250:], tail[-250:]
