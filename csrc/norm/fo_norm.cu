@@ -500,9 +500,12 @@ cudaError_t reorder_launch(const void* X, void* Y, int rows, int dim, int BM, in
   if (rows == 0) return cudaSuccess;
   const int nvec = dim / 8;
   const int vpt = (nvec + kNormThreads - 1) / kNormThreads;
-  // Two rows (what a thread has in flight) per CTA, four where rows are narrow or fill the registers:
-  // 16384 x 8192 2 -> 83.5 us, 4 -> 84.9, 7 -> 89.1; 16384 x 512 2 -> 15.6, 4 -> 13.2; 8192 x 16384 2 -> 106, 4 -> 93.4.
-  const int grid = row_grid(rows, sm_count, vpt == 1 || vpt > 4 ? 4 : 2);
+  // Four rows per CTA, two (what a thread has in flight) for fewer than 24 rows per SM of 2049..8192 elements:
+  // cold, two would be better for any number of those (8192 x 4096: 2 -> 22.1, 4 -> 23.2 us), but not where a
+  // kernel has just written the input and part of it is in the L2 (the two kernels: 2 -> 39.6, 4 -> 37.2 us;
+  // 4096 x 8192: 42.2 and 40.5; 2608 x 8192: 28.7 and 28.1).  Narrow rows and rows that fill the registers want four
+  // either way (16384 x 512: 2 -> 15.6, 4 -> 13.2; 8192 x 16384: 106 and 93.4).
+  const int grid = row_grid(rows, sm_count, vpt == 1 || vpt > 4 || rows >= sm_count * 24 ? 4 : 2);
   const uint16_t* x = static_cast<const uint16_t*>(X);
   uint16_t* y = static_cast<uint16_t*>(Y);
 #define FO_LAUNCH_REORDER(V)                                                                              \
