@@ -141,7 +141,7 @@ enum TraceSlot : int {
   kTraceAccReady = 0,     // epilogue: the tile's accumulator is complete (main loop done)
   kTraceEpilogueDone = 1, // epilogue: last chunk handed to the push warp
   kTracePushIssued = 2,   // push warp: last store of the tile issued
-  kTraceSignalled = 3,    // push warp: stores complete, owners' arrival counters bumped
+  kTraceSignalled = 3,    // signal warp: stores complete, about to bump the owners' arrival counters
   kTraceWaitBegin = 4,    // reducer: starts waiting for the tile's arrivals
   kTraceWaitEnd = 5,      // reducer: every rank's slice has arrived
   kTraceReduced = 6,      // reducer: reduction of the tile issued completely

@@ -1112,8 +1112,9 @@ __global__ void __launch_bounds__(FUSED ? kThreadsFused : kThreadsPlain, 1)
           for (uint32_t j = 0; j < m; ++j) {
             const uint32_t slot = (n + j) % kSigRing;
             const int g = s_sig_g[slot];
-            for (int o = 0; o < p.ws; ++o) ptx::red_relaxed_sys_add(p.flags[(me + o) % p.ws] + g, 1u);
+            // stamped before it is sent: an owner may see it before this lane runs on
             if constexpr (TRACE) stamp(s_sig_t[slot], kTraceSignalled);
+            for (int o = 0; o < p.ws; ++o) ptx::red_relaxed_sys_add(p.flags[(me + o) % p.ws] + g, 1u);
             ptx::mbar_arrive(&sig_empty_bar[slot]);
           }
           n += m;

@@ -7,7 +7,7 @@ AllReduce / ReduceScatter kernels stamp, for every 128-row output tile, eight 64
     0 acc_ready       the tile's accumulator is complete (main loop done)
     1 epilogue_done   last chunk handed to the push warp
     2 push_issued     last store of the tile issued towards the owners
-    3 signalled       the stores have completed and the owners' arrival counters are bumped
+    3 signalled       the stores have completed and the owners' arrival counters are about to be bumped
     4 wait_begin      the owner's reducer starts waiting for the tile
     5 wait_end        every rank's slice has arrived
     6 reduced         the reduction of the tile has been issued completely

@@ -48,3 +48,9 @@ def test_roles_join_their_warps_before_the_cluster_barrier(name, barrier):
     code = _code(name)
     tail = code[:code.rindex(barrier)].rstrip()
     assert "__syncwarp();" in tail[-250:], tail[-250:]
+
+
+def test_a_tile_is_stamped_as_signalled_before_its_owners_can_see_it():
+    code = _code("fo_gemm_sm100.cuh")
+    loop = code[code.index("const int g = s_sig_g[slot]"):code.index("mbar_arrive(&sig_empty_bar[slot])")]
+    assert loop.index("kTraceSignalled") < loop.index("red_relaxed_sys_add")
