@@ -730,7 +730,15 @@ __global__ void __launch_bounds__(FUSED ? kThreadsFused : kThreadsPlain, 1)
           // Accumulator(s) fully read by this warp: hand it back to the (leader's) MMA warp.
           ptx::tc_fence_before_sync();
           __syncwarp();
-          if (lane == 0) ptx::mbar_arrive_cluster(tmem_empty_addr0 + static_cast<uint32_t>(acc) * 8u);
+          if (lane == 0) {
+            // A pair's barrier is the leader's; a CTA by itself signals its own, at its own scope (the emulated
+            // eight ranks of 4096 x 8192 x 1024: 612 us, 696 with the cluster-scope release).
+            if constexpr (CTA2) {
+              ptx::mbar_arrive_cluster(tmem_empty_addr0 + static_cast<uint32_t>(acc) * 8u);
+            } else {
+              ptx::mbar_arrive_cluster_tmem(tmem_empty_addr0 + static_cast<uint32_t>(acc) * 8u);
+            }
+          }
         }
         if constexpr (FUSED) {
           // The buffer is free once the push warp's stores of its previous use have read it.

@@ -26,13 +26,15 @@ def test_tmem_base_is_read_behind_an_ordering_barrier(name):
         assert barriers and barriers[0] in ("__syncthreads", "cluster_arrive_release"), barriers
 
 
-def test_fused_kernel_hands_accumulators_back_at_cluster_scope():
-    """The kernels that run over several GPUs keep the arrive that releases at cluster scope; the CTA-scope
-    form is the plain kernel's."""
+def test_fused_pairs_hand_accumulators_back_at_cluster_scope():
+    """CTA pairs of the kernels that run over several GPUs keep the arrive that releases at cluster scope; the
+    CTA-scope form is the plain kernel's and, on its own barrier, that of a CTA by itself."""
     ptx = re.sub(r"//[^\n]*", "", (GEMM.parent / "common" / "fo_ptx.cuh").read_text())
     body = ptx[ptx.index("void mbar_arrive_cluster("):]
     assert "mbarrier.arrive.release.cluster.shared::cluster" in body[:body.index("}")]
-    assert "mbar_arrive_cluster(" in _code("fo_gemm_sm100.cuh") and "_tmem(" not in _code("fo_gemm_sm100.cuh")
+    fused = re.sub(r"\s+", " ", _code("fo_gemm_sm100.cuh"))
+    assert re.search(r"if constexpr \(CTA2\) \{ ptx::mbar_arrive_cluster\([^;]*\); \} else \{ ptx::mbar_arrive_cluster_tmem\(", fused)
+    assert fused.count("mbar_arrive_cluster") == 2
 
 
 def test_objects_and_launches_query_no_device_properties():
