@@ -124,7 +124,8 @@ def is_tuned(cfg: dict) -> bool:
 
 def is_measured(cfg: dict) -> bool:
     """Whether the config's Algo was timed (a tuner's ``dur``), not picked without a run."""
-    return float(cfg.get("dur", 0.0)) > 0.0
+    dur = cfg.get("dur")
+    return isinstance(dur, (int, float)) and dur > 0
 
 
 def matches(cfg: dict, tp: Optional[int] = None, comm_op: Optional[str] = None, mode: Optional[str] = None) -> bool:

@@ -100,4 +100,5 @@ def test_is_measured(tmp_path):
     path = tmp_path / "cfg.json"
     config.save_solution(path, 128, 256, 0.125, 3, [0, 1], [2])
     assert config.is_measured(config.load_config(path))
-    assert not config.is_measured({"Algo": 3, "BM": 128, "BN": 256, "hint": [0], "cSeg": [1]})
+    for dur in ({}, {"dur": None}, {"dur": [0.1, 0.2]}, {"dur": 0}):
+        assert not config.is_measured({"Algo": 3, "BM": 128, "BN": 256, "hint": [0], "cSeg": [1], **dur})
